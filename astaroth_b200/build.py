@@ -28,11 +28,11 @@ NVCC_FLAGS = ARCH + [
 ]
 CC_FLAGS = ["-O2", "-fPIC", "-fopenmp", "-std=c11", "-Wall", f"-I{INCLUDE}"]
 
-CU_SOURCES = ["device.cu", "device_data.cu", "device_adjoint.cu", "solve.cu", "solve_tiled.cu",
+CU_SOURCES = ["device.cu", "device_data.cu", "device_adjoint.cu", "solve.cu", "solve_tiled.cu", "solve_split.cu",
               "boundconds.cu", "reduce.cu", "cfl.cu", "adjoint.cu", "ensemble.cu", "forcing.cu",
               "bfield.cu", "energy.cu"]
 C_SOURCES = ["host.c"]
-HEADERS = ["internal.h", "mhd_rhs.cuh", "mhd_rhs_adjoint.cuh", "stencil_plain.cuh", "solve_cell.cuh",
+HEADERS = ["internal.h", "mhd_rhs.cuh", "mhd_rhs_adjoint.cuh", "stencil_plain.cuh", "solve_cell.cuh", "pack.cuh",
            "halo.cuh", "tma_ring.cuh", "tmem.cuh", "device_impl.h"]
 
 

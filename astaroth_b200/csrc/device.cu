@@ -102,16 +102,15 @@ ac_make_phys(const AcMeshInfo& info, PhysConst* pc)
 /* The forcing of a substep-2 launch (mhdsolver.ac:531-541): active when
  * AC_lforcing is set and AC_current_time > AC_switch_forcing. */
 /* AC_debug_plain_kernel: 0 = the automatic tiled choice (default), 1 = the plain
- * kernel, 2 = the per-plane tap tiled kernel, 3 = the leading-plane kernel,
- * 4 = the leading-plane kernel with the other group exchange */
+ * kernel, 2 = the per-plane tap tiled kernel, 3 and 4 = the split-stage kernel */
 static int
 solve_variant_of(const AcMeshInfo& info)
 {
     switch (info.int_params[AC_debug_plain_kernel]) {
     case 1: return 0;
     case 2: return AC_SOLVE_TILED_TAPS;
-    case 3: return AC_SOLVE_TILED_LEAD;
-    case 4: return AC_SOLVE_TILED_LEAD_ALT;
+    case 3:
+    case 4: return AC_SOLVE_TILED_SPLIT;
     default: return AC_SOLVE_TILED_AUTO;
     }
 }
@@ -326,6 +325,10 @@ acDeviceCreate(const int id, const AcMeshInfo device_config, Device* device_hand
                  ac_make_tensor_map(&d->tmap[1], d->hi[1], d->geom, precision);
     if (d->tmap_ok)
         CREATE_CHECK(ac_solve_tiled_init(precision));
+    d->split_ok    = ac_make_split_maps(&d->smaps[0], d->hi[0], d->lo[0], d->geom, precision) &&
+                  ac_make_split_maps(&d->smaps[1], d->hi[1], d->lo[1], d->geom, precision);
+    if (d->split_ok)
+        CREATE_CHECK(ac_solve_split_init(precision));
     CREATE_CHECK(cudaMallocHost((void**)&d->host_result, 2 * sizeof(double)));
     CREATE_CHECK(ensure_bfield(d));
     CREATE_CHECK(cudaStreamSynchronize(d->streams[0]));
@@ -783,18 +786,23 @@ launch_substep(Device d, cudaStream_t st, const int step, const double dt,
         }
         cfl = d->cfl;
     }
+    const bool split = tiled && d->split_ok && !pc.upwind && d->solve_variant != AC_SOLVE_TILED_TAPS;
     cudaError_t e;
     if (d->precision == 0) {
         const Fields64 f = fields64(d);
-        e = tiled ? ac_launch_solve_tiled64(d->geom, &d->tmap[blk], f, sc, pc, rk, d->err_flag,
-                                            cfl, st, launches, d->solve_variant)
-                  : ac_launch_solve_plain64(d->geom, f, sc, pc, rk, cfl, st, launches);
+        e = split   ? ac_launch_solve_split64(d->geom, d->smaps[blk], d->smaps[1 - blk], f, sc, pc, rk,
+                                              d->err_flag, cfl, st, launches)
+            : tiled ? ac_launch_solve_tiled64(d->geom, &d->tmap[blk], f, sc, pc, rk, d->err_flag,
+                                              cfl, st, launches)
+                    : ac_launch_solve_plain64(d->geom, f, sc, pc, rk, cfl, st, launches);
     }
     else {
         const Fields32 f = fields32(d);
-        e = tiled ? ac_launch_solve_tiled32(d->geom, &d->tmap[blk], f, sc, pc, rk, d->err_flag,
-                                            cfl, st, launches, d->solve_variant)
-                  : ac_launch_solve_plain32(d->geom, f, sc, pc, rk, cfl, st, launches);
+        e = split   ? ac_launch_solve_split32(d->geom, d->smaps[blk], d->smaps[1 - blk], f, sc, pc, rk,
+                                              d->err_flag, cfl, st, launches)
+            : tiled ? ac_launch_solve_tiled32(d->geom, &d->tmap[blk], f, sc, pc, rk, d->err_flag,
+                                              cfl, st, launches)
+                    : ac_launch_solve_plain32(d->geom, f, sc, pc, rk, cfl, st, launches);
     }
     if (e != cudaSuccess || !pc.forcing)
         return e;

@@ -174,6 +174,8 @@ struct ensemble_s {
     /* mode 1: per-member tensor maps of both buffer parities, branch streams */
     std::vector<CUtensorMap> tmaps; /* 2 per member: [2 m + parity] */
     std::vector<char> tiled;        /* member fits the tiled kernel (else: plain) */
+    std::vector<SplitBufferMaps> smaps; /* 2 per member, of the split-stage kernel */
+    std::vector<char> split;            /* member fits it */
     std::vector<cudaStream_t> branches;
     std::vector<cudaEvent_t> joins;
     cudaEvent_t fork;
@@ -328,6 +330,13 @@ build_items(Ensemble e, const AcEnsembleTiles t)
     return cudaSuccess;
 }
 
+/* whether a step runs as one launch per member and substep */
+bool
+per_member(const AcEnsembleTiles& t)
+{
+    return t.mode == 1 || t.blocks_per_sm == AC_ENSEMBLE_MEMBER_LAUNCHES;
+}
+
 bool
 tiles_ok(const AcEnsembleTiles t)
 {
@@ -379,7 +388,7 @@ launch_halo(Ensemble e, unsigned long long* launches)
 template <typename T, bool COMP>
 cudaError_t
 record_members(Ensemble e, const int s0, const int s1, unsigned long long* launches,
-               const bool halo = true)
+               const bool exact, const bool halo = true)
 {
     cudaError_t err = cudaEventRecord(e->fork, e->stream);
     if (err != cudaSuccess)
@@ -411,19 +420,32 @@ record_members(Ensemble e, const int s0, const int s1, unsigned long long* launc
             }
             const RkCoef rk     = ac_rk_coef(s, e->dts[m]);
             const void* tmap    = &e->tmaps[2 * m + p];
-            /* the kernel a Device of this member would use */
+            /* the kernel a Device of this member would use, or (exact) one with the
+             * plain kernel's bits.  The members of the
+             * other branches run beside it: its z chunks are chosen for its share
+             * of the SMs (longer chunks, less work on halo planes) */
+            const int sms               = std::max(1, AC_SMS / nb);
+            const SplitBufferMaps& smi = e->smaps[2 * m + p];
+            const SplitBufferMaps& smo = e->smaps[2 * m + (p ^ 1)];
+            const bool split = e->split[m] && !exact;
             if constexpr (COMP)
-                err = e->tiled[m] ? ac_launch_solve_tiled32(r.g, tmap, f, e->sc[m], e->pc[m], rk,
-                                                            e->err, nullptr, st, launches,
-                                                            AC_SOLVE_TILED_AUTO)
-                                  : ac_launch_solve_plain32(r.g, f, e->sc[m], e->pc[m], rk, nullptr,
-                                                            st, launches);
+                err = split
+                          ? ac_launch_solve_split32(r.g, smi, smo, f, e->sc[m], e->pc[m], rk, e->err,
+                                                    nullptr, st, launches, sms)
+                      : e->tiled[m]
+                          ? ac_launch_solve_tiled32(r.g, tmap, f, e->sc[m], e->pc[m], rk, e->err,
+                                                    nullptr, st, launches)
+                          : ac_launch_solve_plain32(r.g, f, e->sc[m], e->pc[m], rk, nullptr, st,
+                                                    launches);
             else
-                err = e->tiled[m] ? ac_launch_solve_tiled64(r.g, tmap, f, e->sc[m], e->pc[m], rk,
-                                                            e->err, nullptr, st, launches,
-                                                            AC_SOLVE_TILED_AUTO)
-                                  : ac_launch_solve_plain64(r.g, f, e->sc[m], e->pc[m], rk, nullptr,
-                                                            st, launches);
+                err = split
+                          ? ac_launch_solve_split64(r.g, smi, smo, f, e->sc[m], e->pc[m], rk, e->err,
+                                                    nullptr, st, launches, sms)
+                      : e->tiled[m]
+                          ? ac_launch_solve_tiled64(r.g, tmap, f, e->sc[m], e->pc[m], rk, e->err,
+                                                    nullptr, st, launches)
+                          : ac_launch_solve_plain64(r.g, f, e->sc[m], e->pc[m], rk, nullptr, st,
+                                                    launches);
             if (err != cudaSuccess)
                 return err;
         }
@@ -442,9 +464,11 @@ record_members(Ensemble e, const int s0, const int s1, unsigned long long* launc
 cudaError_t
 record_step(Ensemble e, unsigned long long* launches)
 {
-    if (e->tiles.mode == 1) {
-        const cudaError_t err = e->precision == 0 ? record_members<double, false>(e, 0, 3, launches)
-                                                  : record_members<float, true>(e, 0, 3, launches);
+    if (per_member(e->tiles)) {
+        const bool exact      = e->tiles.mode == 0;
+        const cudaError_t err = e->precision == 0
+                                    ? record_members<double, false>(e, 0, 3, launches, exact)
+                                    : record_members<float, true>(e, 0, 3, launches, exact);
         if (err == cudaSuccess)
             e->parity ^= 1; /* three swaps */
         return err;
@@ -685,14 +709,21 @@ acEnsembleCreate(const int device_id, const int n, const AcMeshInfo* member_info
     ENS_CHECK(cudaMemset(e->err, 0, sizeof(int)));
     e->tmaps.resize(2 * (size_t)n);
     e->tiled.assign(n, 1);
+    e->smaps.resize(2 * (size_t)n);
+    e->split.assign(n, 1);
     for (int m = 0; m < n; ++m)
         for (int p = 0; p < 2; ++p) {
             void* base = e->precision == 0 ? (void*)members<double>(e)[m].f[p].in[0]
                                            : (void*)members<float>(e)[m].f[p].in[0];
+            float* lo  = e->precision == 0 ? nullptr
+                                           : const_cast<float*>(members<float>(e)[m].f[p].in_lo[0]);
             if (!ac_make_tensor_map(&e->tmaps[2 * m + p], base, e->geom[m], e->precision))
                 e->tiled[m] = 0;
+            if (!ac_make_split_maps(&e->smaps[2 * m + p], base, lo, e->geom[m], e->precision))
+                e->split[m] = 0;
         }
     ENS_CHECK(ac_solve_tiled_init(e->precision));
+    ENS_CHECK(ac_solve_split_init(e->precision));
     const int nb = std::min(n, 16);
     e->branches.assign(nb, nullptr);
     e->joins.assign(nb, nullptr);
@@ -828,7 +859,7 @@ acEnsembleIntegrateStep(const Ensemble e)
         e->graph_valid[pc] = 1;
     }
     AC_CUDA_CHECK(cudaGraphLaunch(e->graph[p], e->stream));
-    e->launches += e->tiles.mode == 1 ? 6ull * e->n : 6ull; /* halo + solve, 3 substeps */
+    e->launches += per_member(e->tiles) ? 6ull * e->n : 6ull; /* halo + solve, 3 substeps */
     e->parity ^= 1; /* three swaps */
     return AC_SUCCESS;
 }
@@ -931,19 +962,24 @@ acEnsembleAutotune(const Ensemble e, AcEnsembleTiles* best, double* best_ms)
             win    = t;
         }
     }
-    /* then the two modes on the solve of substep 0 (no halo fill, so the state
-     * is left as it was), each replayed from a captured graph */
-    auto time_graph = [&](const int mode, double* ms) -> cudaError_t {
+    /* then the forms of a step on the solve of substep 0 (no halo fill, so the
+     * state is left as it was), each replayed from a captured graph: the
+     * persistent launch, one launch per member with the same bits, and mode 1
+     * where some member is past the sizes of the tap kernel (an ensemble of small
+     * members keeps the bits of its sequential launches) */
+    enum { PERSISTENT, MEMBERS, MODE1 };
+    auto time_graph = [&](const int form, double* ms) -> cudaError_t {
         cudaGraph_t graph;
         cudaGraphExec_t exec;
         cudaError_t rec = cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal);
         if (rec != cudaSuccess)
             return rec;
-        if (mode == 0)
+        if (form == PERSISTENT)
             rec = launch_solve(e, 0, NULL);
         else
-            rec = e->precision == 0 ? record_members<double, false>(e, 0, 1, NULL, false)
-                                    : record_members<float, true>(e, 0, 1, NULL, false);
+            rec = e->precision == 0
+                      ? record_members<double, false>(e, 0, 1, NULL, form == MEMBERS, false)
+                      : record_members<float, true>(e, 0, 1, NULL, form == MEMBERS, false);
         const cudaError_t end = cudaStreamEndCapture(e->stream, &graph);
         if (rec != cudaSuccess)
             return rec;
@@ -969,16 +1005,22 @@ acEnsembleAutotune(const Ensemble e, AcEnsembleTiles* best, double* best_ms)
     };
     if (err == cudaSuccess)
         err = build_items(e, win);
-    double ms0 = 0, ms1 = 1e300;
-    if (err == cudaSuccess)
-        err = time_graph(0, &ms0);
-    if (err == cudaSuccess)
-        err = time_graph(1, &ms1);
+    bool large = false;
+    for (int m = 0; m < e->n; ++m)
+        large = large || ac_taps_zchunk(e->geom[m], e->precision) >= 32;
+    double ms[3] = {1e300, 1e300, 1e300};
+    for (int form = PERSISTENT; form <= (large ? MODE1 : MEMBERS) && err == cudaSuccess; ++form)
+        err = time_graph(form, &ms[form]);
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
     AC_CUDA_CHECK(err);
-    win.mode = ms1 < ms0 ? 1 : 0;
-    win_ms   = ms1 < ms0 ? ms1 : ms0;
+    const int form = ms[MODE1] < std::min(ms[PERSISTENT], ms[MEMBERS]) ? MODE1
+                     : ms[MEMBERS] < ms[PERSISTENT]                     ? MEMBERS
+                                                                        : PERSISTENT;
+    win.mode = form == MODE1;
+    if (form == MEMBERS)
+        win.blocks_per_sm = AC_ENSEMBLE_MEMBER_LAUNCHES;
+    win_ms = ms[form];
     AC_CUDA_CHECK(build_items(e, win));
     if (best)
         *best = win;

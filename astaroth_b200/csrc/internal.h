@@ -12,7 +12,8 @@
 
 #include "astaroth_b200.h"
 
-#define AC_NF 8 /* number of fields of the MHD module */
+#define AC_NF 8    /* number of fields of the MHD module */
+#define AC_SMS 148 /* SMs of a B200 */
 
 /* Report a CUDA error and return AC_FAILURE from the calling API function. */
 #define AC_CUDA_CHECK(call)                                                                   \
@@ -148,10 +149,19 @@ struct StepGraph {
     int valid;
 };
 
+/* The split-stage kernel (solve_split.cu): tensor maps of one buffer block, of
+ * its values with the tile's halo and of the tile alone (values, FP32
+ * compensation words). */
+struct SplitBufferMaps {
+    CUtensorMap plane, tile, tile_lo;
+};
+
 /* The two buffers of every field: block b holds all 8 fields of buffer b
  * (field q at offset q*cells).  in_idx[q] says which block is field q's
  * in-buffer; swaps flip it. */
 struct device_s {
+    SplitBufferMaps smaps[2]; /* the split-stage kernel's maps of each block */
+    int split_ok;
     CUtensorMap tmap[2]; /* 4-D (x, y, z, field) maps of the value (hi) array of each block */
     int tmap_ok;
     int* err_flag;       /* device word set by kernels whose bounded waits gave up */
@@ -269,29 +279,42 @@ cudaError_t ac_launch_reduce(const Geom& g, const void* const* fields, const flo
 
 int ac_reduce_blocks(const Geom& g);
 
-/* Tiled substep kernels (solve_tiled.cu): the leading-plane kernel (in-plane
- * derivatives of plane z+3 kept in tensor memory until plane z is solved) and
- * the per-plane tap kernel.  AUTO takes the leading-plane kernel for z chunks
- * of 32 planes and more; _ALT is the leading-plane kernel with the group
- * exchange through shared memory instead of tensor memory.  Meshes with the
- * upwinding terms always take the per-plane tap kernel. */
+/* Tiled substep kernels: the split-stage kernel (solve_split.cu), which the
+ * automatic choice takes for every mesh it fits, and the per-plane tap kernel
+ * (solve_tiled.cu) for the upwinding terms and for the others. */
 enum {
-    AC_SOLVE_TILED_AUTO     = 1,
-    AC_SOLVE_TILED_TAPS     = 2,
-    AC_SOLVE_TILED_LEAD     = 3,
-    AC_SOLVE_TILED_LEAD_ALT = 4
+    AC_SOLVE_TILED_AUTO  = 1,
+    AC_SOLVE_TILED_TAPS  = 2,
+    AC_SOLVE_TILED_SPLIT = 3
 };
+/* false where the kernel does not take the mesh */
+bool ac_make_split_maps(SplitBufferMaps* m, void* hi, float* lo, const Geom& g,
+                        const int precision);
+cudaError_t ac_solve_split_init(const int precision);
+/* sms: SMs that this launch can expect to have (fewer where others run beside it) */
+cudaError_t ac_launch_solve_split64(const Geom& g, const SplitBufferMaps& in,
+                                    const SplitBufferMaps& out, const Fields64& f,
+                                    const StencilCoef& sc, const PhysConst& pc, const RkCoef& rk,
+                                    int* err, unsigned long long* cfl, cudaStream_t stream,
+                                    unsigned long long* launches, const int sms = AC_SMS);
+cudaError_t ac_launch_solve_split32(const Geom& g, const SplitBufferMaps& in,
+                                    const SplitBufferMaps& out, const Fields32& f,
+                                    const StencilCoef& sc, const PhysConst& pc, const RkCoef& rk,
+                                    int* err, unsigned long long* cfl, cudaStream_t stream,
+                                    unsigned long long* launches, const int sms = AC_SMS);
+/* the z chunk that the tap kernel takes for a whole mesh: 32 and more above about 96^3 */
+int ac_taps_zchunk(const Geom& g, const int precision);
 bool ac_tiled_supported(const Geom& g, const int precision);
 bool ac_make_tensor_map(void* map_out, void* base, const Geom& g, const int precision);
 cudaError_t ac_solve_tiled_init(const int precision);
 cudaError_t ac_launch_solve_tiled64(const Geom& g, const void* tmap_in, const Fields64& f,
                                     const StencilCoef& sc, const PhysConst& pc, const RkCoef& rk,
                                     int* err, unsigned long long* cfl, cudaStream_t stream,
-                                    unsigned long long* launches, const int kernel);
+                                    unsigned long long* launches);
 cudaError_t ac_launch_solve_tiled32(const Geom& g, const void* tmap_in, const Fields32& f,
                                     const StencilCoef& sc, const PhysConst& pc, const RkCoef& rk,
                                     int* err, unsigned long long* cfl, cudaStream_t stream,
-                                    unsigned long long* launches, const int kernel);
+                                    unsigned long long* launches);
 
 /* Helical forcing added to the three velocity arrays u (and their
  * compensation arrays lo in FP32) after substep 2 (forcing.cu). */

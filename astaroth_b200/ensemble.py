@@ -8,9 +8,10 @@ without tiling, so a member's result equals that Device's bit for bit.
 
 The tile shape of the persistent launch comes from ``Ensemble.autotune``: the
 library times a fixed candidate set on the current members, then compares a
-whole substep of the best persistent launch with mode 1 (one shared-memory
-tiled launch per member, the members' launches as concurrent graph branches)
-and keeps the faster; the result can be cached in a JSON file keyed by the
+whole substep of the best persistent launch with one tap-kernel launch per
+member (the same bits, the members' launches as concurrent graph branches) and,
+where some member is larger than about 96^3, with mode 1 (the launches of the
+members' own Devices), and keeps the fastest; the result can be cached in a JSON file keyed by the
 member sizes, the precision and the GPU name.
 """
 from __future__ import annotations
@@ -132,7 +133,8 @@ class Ensemble:
 
     def set_tiles(self, tx: int, ty: int, zb: int, blocks_per_sm: int = 0, mode: int = 0) -> None:
         """mode 0: persistent work-list solve with these tiles; mode 1: concurrent
-        per-member tiled launches (the tiles still describe mode 0's work list)."""
+        launches per member of the kernel its own Device uses, the fastest form
+        (the tiles still describe mode 0's work list)."""
         _check(self.lib.acEnsembleSetTiles(self._h, AcEnsembleTiles(tx, ty, zb, blocks_per_sm,
                                                                     mode)),
                "acEnsembleSetTiles")

@@ -563,7 +563,7 @@ def ensemble_leg(args, torch, rank, world):
     modes = {}
     for mode in (0, 1):
         try:
-            e.set_tiles(*tiles[:4], mode=mode)
+            e.set_tiles(*tiles[:3], mode=mode)
         except Exception:
             continue
         for _ in range(args.warmup):

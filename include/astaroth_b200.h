@@ -778,13 +778,15 @@ typedef struct ensemble_s* Ensemble;
 
 /* How a step runs.  mode 0: the persistent solve over the work list: tx * ty
  * threads per block (one cell per thread and plane), zb planes per work item,
- * blocks_per_sm resident blocks per SM (0 = the occupancy limit).  mode 1:
- * one launch per member and substep of the kernel a single-mesh Device of
- * that member uses (the tiled shared-memory plane-ring kernel, or the plain one
- * for meshes it does not fit), the members' launch chains as concurrent
- * branches of the step graph (tx, ty, zb, blocks_per_sm unused).  Both give
- * each member the bits of a single-mesh Device of that member (mode 0: of its
- * plain kernel; mode 1: of its default kernel). */
+ * blocks_per_sm resident blocks per SM (0 = the occupancy limit), or, with
+ * blocks_per_sm = AC_ENSEMBLE_MEMBER_LAUNCHES, one launch per member and substep
+ * of the tap kernel, which has the same bits, as concurrent branches of the
+ * step graph.  mode 1: one launch per member and substep of the kernel a
+ * single-mesh Device of that member uses (the split-stage kernel, or the tap or
+ * plain one for meshes it does not fit), as such branches (tx, ty, zb,
+ * blocks_per_sm unused).  Each member gets the bits of a single-mesh Device of
+ * that member (mode 0: of its plain kernel; mode 1: of its default kernel). */
+#define AC_ENSEMBLE_MEMBER_LAUNCHES 1048576
 typedef struct {
     int tx, ty, zb, blocks_per_sm;
     int mode;
@@ -809,8 +811,12 @@ AcResult acEnsembleIntegrateStepSequential(const Ensemble ensemble);
 AcResult acEnsembleSetTiles(const Ensemble ensemble, const AcEnsembleTiles tiles);
 AcResult acEnsembleGetTiles(const Ensemble ensemble, AcEnsembleTiles* tiles);
 /* Times the solve of substep 0 (which leaves the in-buffers unchanged) for
- * the persistent launch over a fixed candidate set of tiles, then for mode 1,
- * keeps the fastest and returns it with its time per substep in milliseconds. */
+ * the persistent launch over a fixed candidate set of tiles, then for the
+ * launches per member of mode 0 and, where some member is larger than about
+ * 96^3, of mode 1, keeps the fastest and returns it with its time per substep in
+ * milliseconds.  (Ensembles of small members so keep the bits of their
+ * sequential launches; mode 1 is faster and can be set where these are not
+ * needed.) */
 AcResult acEnsembleAutotune(const Ensemble ensemble, AcEnsembleTiles* best, double* best_ms);
 /* Reduction of one member's in-buffer, as acDeviceReduceScal / acDeviceReduceVec. */
 AcResult acEnsembleReduceScal(const Ensemble ensemble, const int member, const AcReduction reduction,

@@ -1,0 +1,66 @@
+"""The split-stage substep kernel (the automatic choice) against the plain kernel
+at the sizes where its tiles, chunks and queues have their edges: one tile and
+one cell more or less, chunks of a few planes, rows of the packed FP32 tile that
+lie outside the mesh.  Both evaluate the same equations with their sums in
+another order.
+
+Tolerances: per step a field changes by at most dt |rate|, and the two sums of a
+rate differ by at most a few hundred roundings (the terms of the stencils and of
+the equations) of its largest term.  With dt |term| <= 0.05 max|f| here and
+2 steps of 3 substeps, FP64 stays within 6 * 0.05 * 300 * 1.1e-16 < 1e-14 of
+max|f|; FP32 rates within 6 * 0.05 * 300 * 6e-8 < 6e-6."""
+import numpy as np
+import pytest
+
+from astaroth_b200 import capi
+from astaroth_b200.device import CONFIG_PARAMS, Device, make_info, seeded_mesh
+
+pytestmark = pytest.mark.gpu
+
+AMP = dict(amp_scalar=1e-2, sigma_uu=3e-2, sigma_aa=3e-3)
+SIZES = [(32, 4, 3), (32, 8, 8), (34, 7, 5), (62, 9, 4), (66, 16, 11), (96, 12, 37), (150, 13, 17)]
+
+
+def run(n, precision, kernel, **params):
+    info = make_info(n, precision=precision, **dict(CONFIG_PARAMS, **params))
+    info.int_params[capi.IntParam.AC_debug_plain_kernel] = kernel
+    f = seeded_mesh(info, 17, **AMP)
+    with Device(info) as d:
+        d.load_mesh(f)
+        for _ in range(2):
+            d.integrate_step(1e-3)
+        d.synchronize()
+        return d.store_mesh()[:, 3:-3, 3:-3, 3:-3].copy(), d.timestep_maxima(), d.timestep()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", SIZES)
+def test_split_kernel_equals_plain(n, precision):
+    a, ma, _ = run(n, precision, 1)
+    b, mb, _ = run(n, precision, 0)
+    scale = np.abs(a).reshape(8, -1).max(axis=1)
+    err = np.abs(a - b).reshape(8, -1).max(axis=1) / scale
+    assert err.max() <= (1e-14 if precision == 0 else 6e-6), err
+    np.testing.assert_allclose(ma, mb, rtol=1e-13 if precision == 0 else 6e-6)
+
+
+def test_z_boxes_of_any_size_give_the_same_bits():
+    """Chunks start and end anywhere: the planes of a substep solved in uneven z boxes."""
+    n = (40, 12, 19)
+    info = make_info(n, **CONFIG_PARAMS)
+    f = seeded_mesh(info, 5, **AMP)
+    out = []
+    for cuts in ((0, 19), (0, 1, 3, 4, 11, 19), (0, 6, 13, 19)):
+        with Device(info) as d:
+            d.load_mesh(f)
+            for s in range(3):
+                d.periodic_boundconds()
+                for z0, z1 in zip(cuts, cuts[1:]):
+                    assert d.lib.acDeviceIntegrateSubstep(
+                        d.handle, 0, s, capi.Volume(3, 3, 3 + z0),
+                        capi.Volume(3 + n[0], 3 + n[1], 3 + z1), 1e-3) == 0
+                d.swap_buffers()
+            d.synchronize()
+            out.append((d.store_mesh(), d.timestep_maxima()))
+    for o, m in out[1:]:
+        assert np.array_equal(o, out[0][0]) and m == out[0][1]
