@@ -281,7 +281,7 @@ int ac_reduce_blocks(const Geom& g);
 
 /* Tiled substep kernels: the split-stage kernel (solve_split.cu), which the
  * automatic choice takes for every mesh it fits, and the per-plane tap kernel
- * (solve_tiled.cu) for the upwinding terms and for the others. */
+ * (solve_tiled.cu) for the others. */
 enum {
     AC_SOLVE_TILED_AUTO  = 1,
     AC_SOLVE_TILED_TAPS  = 2,

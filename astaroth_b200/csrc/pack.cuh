@@ -82,6 +82,16 @@ operator-(const F2 a)
     return F2{a.v ^ 0x8000000080000000ull};
 }
 __device__ __forceinline__ F2
+vabs(const F2 a)
+{
+    return F2{a.v & 0x7fffffff7fffffffull};
+}
+__device__ __forceinline__ double
+vabs(const double a)
+{
+    return fabs(a);
+}
+__device__ __forceinline__ F2
 ac_exp(const F2 a)
 {
     return f2(ac_exp(lo_of(a)), ac_exp(hi_of(a)));

@@ -133,6 +133,7 @@ struct SplitCoef {
     V mm[3][3]; /* mix / mu0 */
     V mmn[2][3];
     V nim;      /* -1/mu0 */
+    V up[3][4]; /* upwinding, [axis][k]: centre and sides */
     /* equations */
     V m23, two, one_half, two_nu, nu, inv_cp, ncs2, gicp, gm1, gm1_lnrho0, inv_exp_lnT0, eta, eta_mu0,
         zeta, K;
@@ -159,6 +160,8 @@ make_coef(const StencilCoef& s, const PhysConst& p)
             }
         }
         c.d2c[a] = D(s.d2[a][0]);
+        for (int k = 0; k < 4; ++k)
+            c.up[a][k] = D(s.up[a][k]);
         c.vc[a]  = D(nu * ((long double)s.d2[0][0] + s.d2[1][0] + s.d2[2][0]) + vg * s.d2[a][0]);
     }
     c.c_all = D((long double)s.d2[0][0] + s.d2[1][0] + s.d2[2][0]);
@@ -229,23 +232,27 @@ enum {
     M_DYAZ,
     REC_N
 };
-constexpr int REC_HN = M_SX;          /* the hydro group's part */
-constexpr int REC_MN = REC_N - M_SX;    /* the magnetic group's part */
+constexpr int REC_MN = REC_N - M_SX; /* the magnetic group's part */
 constexpr int HX_N = 7;               /* exchange: grad lnrho, lap lnrho, 2 S:S, div u, exp(-lnrho) */
 constexpr int MX_N = 10; /* grad s, j, B, exp(gamma s/cp + (gamma-1)(lnrho - lnrho0)) */
 
 constexpr uint32_t REC_SLOTS = 5, Q_SLOTS = 8;
-constexpr uint32_t REC_W = 2 * REC_N;
-constexpr uint32_t ACC0  = REC_SLOTS * REC_W;
-constexpr uint32_t ACC_W = 2 * 6;              /* three sums per group */
-constexpr uint32_t ZQ0   = ACC0 + 2 * ACC_W;
-constexpr uint32_t ZQ_W  = 2 * 4;              /* one plane's four values */
-constexpr uint32_t ZQ_G  = Q_SLOTS * ZQ_W;     /* one group's queue */
-constexpr uint32_t XCH0  = ZQ0 + 2 * ZQ_G;
-constexpr uint32_t XCH_W = 2 * (HX_N + MX_N);
-constexpr uint32_t TM_END = XCH0 + 2 * XCH_W;
+constexpr uint32_t ACC_W   = 2 * 6;            /* mixed sums of a plane: three per group */
+constexpr uint32_t ZQ_W    = 2 * 4;            /* one plane's four values */
+constexpr uint32_t ZQ_G    = Q_SLOTS * ZQ_W;   /* one group's queue */
+constexpr uint32_t XCH_W   = 2 * (HX_N + MX_N);
 constexpr uint32_t TM_COLS = 512;
-static_assert(TM_END <= TM_COLS, "tensor-memory columns");
+/* UPWD: the hydro record also has the in-plane upwinding terms |ux| d_x + |uy| d_y
+ * of lnrho, ux, uy, uz behind the values above */
+template <bool UPWD>
+struct Tm {
+    static constexpr int HN         = M_SX + (UPWD ? 4 : 0); /* the hydro group's part */
+    static constexpr uint32_t REC_W = 2 * (HN + REC_MN);
+    static constexpr uint32_t ACC0  = REC_SLOTS * REC_W;
+    static constexpr uint32_t ZQ0   = ACC0 + 2 * ACC_W;
+    static constexpr uint32_t XCH0  = ZQ0 + 2 * ZQ_G;
+    static_assert(XCH0 + 2 * XCH_W <= TM_COLS, "tensor-memory columns");
+};
 
 /* ---- shared memory ---- */
 
@@ -401,7 +408,7 @@ load_prev(const SplitMaps* maps, const Chunk& ch, typename Pack<V>::T* smem, con
 /* ---------------------------------------------------------------------------
  * The in-plane roles.
  * ------------------------------------------------------------------------- */
-template <typename V, int GROUP>
+template <typename V, int GROUP, bool UPWD>
 __device__ __forceinline__ bool
 inplane_role(const SplitMaps* maps, const SplitCoef<V>& c, const Chunk& ch,
              typename Pack<V>::T* smem, const int cell_off, const bool loader, const bool use_prev,
@@ -420,7 +427,8 @@ inplane_role(const SplitMaps* maps, const SplitCoef<V>& c, const Chunk& ch,
             acc[a][j] = Pack<V>::dup(0.0);
     int slot = 0;
     unsigned phase = 0;
-    uint32_t rec = ch.tl + (GROUP == 0 ? 0u : 2u * M_SX); /* record slot, stepped with the plane */
+    typedef Tm<UPWD> TM;
+    uint32_t rec = ch.tl + (GROUP == 0 ? 0u : 2u * TM::HN); /* record slot, stepped with the plane */
     uint32_t r5  = 0;
     /* (the first plane takes record slot 0: the solve roles count alike) */
 #pragma unroll 1
@@ -441,22 +449,32 @@ inplane_role(const SplitMaps* maps, const SplitCoef<V>& c, const Chunk& ch,
         if (L >= ch.z0 && L < ch.z1) {
             V dx[3], sx[3], dy[3], sy[3];
             if constexpr (GROUP == 0) {
-                TWords<REC_HN> r;
+                TWords<TM::HN> r;
+                [[maybe_unused]] const V au = vabs(v0), av = vabs(v1);
+                auto upwind = [&](const int q, const V v) {
+                    if constexpr (UPWD)
+                        r.set(M_SX + q, vfma(au, dot3p(sx, &c.up[0][1], c.up[0][0] * v),
+                                             av * dot3p(sy, &c.up[1][1], c.up[1][0] * v)));
+                };
                 taps_xy(ts, dx, sx, dy, sy);
+                upwind(0, vs);
                 r.set(H_SX, dot3(dx, c.d1[0]));
                 r.set(H_SY, dot3(dy, c.d1[1]));
                 r.set(H_SL, dot3p(sy, c.d2[1], dot3p(sx, c.d2[0], c.c_all * vs)));
                 taps_xy(t0, dx, sx, dy, sy);
+                upwind(1, v0);
                 const V done = mixed_first(acc[2], dx, e1, n1);
                 r.set(H_C + 0, dot3(dx, c.d1[0]));
                 r.set(H_C + 1, dot3(dy, c.d1[1]));
                 r.set(H_C + 2, dxy(t1, c.vm[0], dot3p(sy, c.vn[1], dot3p(sx, c.vd[0], c.vc[0] * v0))));
                 taps_xy(t1, dx, sx, dy, sy);
+                upwind(2, v1);
                 fin.set(2, mixed_second(acc[2], done, dy, e2, n2));
                 r.set(H_C + 3, dot3(dx, c.d1[0]));
                 r.set(H_C + 4, dot3(dy, c.d1[1]));
                 r.set(H_C + 5, dxy(t0, c.vm[0], dot3p(sy, c.vd[1], dot3p(sx, c.vn[0], c.vc[1] * v1))));
                 taps_xy(t2, dx, sx, dy, sy);
+                upwind(3, v2);
                 fin.set(0, mixed_first(acc[0], dx, e1, n1));
                 fin.set(1, mixed_first(acc[1], dy, e2, n2));
                 r.set(H_C + 6, dot3(dx, c.d1[0]));
@@ -511,14 +529,14 @@ inplane_role(const SplitMaps* maps, const SplitCoef<V>& c, const Chunk& ch,
             fin.set(1, mixed_first(acc[1], e, e2, n2));
             __syncwarp();
         }
-        fin.store(ch.tl + ACC0 + (uint32_t)((L - NGHOST) & 1) * ACC_W + GROUP * 6u);
+        fin.store(ch.tl + TM::ACC0 + (uint32_t)((L - NGHOST) & 1) * ACC_W + GROUP * 6u);
         {
             TWords<4> q;
             q.set(0, vs);
             q.set(1, v0);
             q.set(2, v1);
             q.set(3, v2);
-            q.store(ch.tl + ZQ0 + GROUP * ZQ_G + (uint32_t)(L & 7) * ZQ_W);
+            q.store(ch.tl + TM::ZQ0 + GROUP * ZQ_G + (uint32_t)(L & 7) * ZQ_W);
         }
         interval_end();
         if (loader) {
@@ -537,7 +555,7 @@ inplane_role(const SplitMaps* maps, const SplitCoef<V>& c, const Chunk& ch,
             slot = 0;
             phase ^= 1;
         }
-        rec = ++r5 == REC_SLOTS ? (r5 = 0, rec - (REC_SLOTS - 1) * REC_W) : rec + REC_W;
+        rec = ++r5 == REC_SLOTS ? (r5 = 0, rec - (REC_SLOTS - 1) * TM::REC_W) : rec + TM::REC_W;
     }
     interval_end(); /* the last solve interval's exchange */
     return ok;
@@ -556,6 +574,18 @@ z_derivs(const TWords<4> w[7], const int i, const V d1[3], const V d2[3], V& g, 
     const V p1 = w[4].template get<V>(i), p2 = w[5].template get<V>(i), p3 = w[6].template get<V>(i);
     g = vfma(d1[2], p3 - m3, vfma(d1[1], p2 - m2, d1[0] * (p1 - m1)));
     s = vfma(d2[2], p3 + m3, vfma(d2[1], p2 + m2, d2[0] * (p1 + m1)));
+}
+
+/* the upwinding derivative along z */
+template <typename V>
+__device__ __forceinline__ V
+z_upwind(const TWords<4> w[7], const int i, const V u[4])
+{
+    V r = u[0] * w[3].template get<V>(i);
+#pragma unroll
+    for (int k = 1; k <= 3; ++k)
+        r = vfma(u[k], w[3 + k].template get<V>(i) + w[3 - k].template get<V>(i), r);
+    return r;
 }
 
 template <typename V>
@@ -638,7 +668,7 @@ cfl_cells(const F2 u2, const F2 b2, const F2 irho, const float cs2, float m[3], 
         cfl_accumulate(hi_of(u2), hi_of(b2), hi_of(irho), cs2, m, with_sum);
 }
 
-template <typename V, int GROUP, bool PREV>
+template <typename V, int GROUP, bool PREV, bool UPWD>
 __device__ __forceinline__ bool
 solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitCoef<V>& c,
            const RkV<V>& rk, const Chunk& ch, const typename Pack<V>::T* prev, const int lx,
@@ -657,9 +687,10 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
         prev + 4 * GROUP * S::PFLD + ly * S::PXW + lx + (NGHOST - S::PX0);
     int pslot       = 0;
     unsigned pphase = 0;
-    const uint32_t zq = ch.tl + ZQ0 + GROUP * ZQ_G;
+    typedef Tm<UPWD> TM;
+    const uint32_t zq = ch.tl + TM::ZQ0 + GROUP * ZQ_G;
     uint32_t r5 = 3 % REC_SLOTS; /* record slot of plane z0 = pfirst + 3 */
-    uint32_t rec = ch.tl + r5 * REC_W;
+    uint32_t rec = ch.tl + r5 * TM::REC_W;
 #pragma unroll 1
     for (int i = 0; i < 7; ++i)
         interval_end();
@@ -673,11 +704,11 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
 #pragma unroll
         for (int k = 0; k < 7; ++k)
             w[k].tie();
-        const uint32_t xslot = ch.tl + XCH0 + (uint32_t)(p & 1) * XCH_W;
-        const uint32_t aslot = ch.tl + ACC0 + (uint32_t)(p & 1) * ACC_W + GROUP * 6u;
+        const uint32_t xslot = ch.tl + TM::XCH0 + (uint32_t)(p & 1) * XCH_W;
+        const uint32_t aslot = ch.tl + TM::ACC0 + (uint32_t)(p & 1) * ACC_W + GROUP * 6u;
         V val[4], rr[4];
         if constexpr (GROUP == 0) {
-            TWords<REC_HN> r;
+            TWords<TM::HN> r;
             TWords<3> a;
             r.load(rec);
             a.load(aslot);
@@ -688,9 +719,21 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
             z_derivs(w, 1, c.d1[2], c.vn[2], gz[0], s2[1]);
             z_derivs(w, 2, c.d1[2], c.vn[2], gz[1], s2[2]);
             z_derivs(w, 3, c.d1[2], c.vd[2], gz[2], s2[3]);
+            [[maybe_unused]] V upz[4];
+            if constexpr (UPWD) {
+                const V aw = vabs(uz);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    upz[q] = aw * z_upwind(w, q, c.up[2]);
+            }
             tmem::wait_ld();
             r.tie();
             a.tie();
+            if constexpr (UPWD) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    upz[q] = upz[q] + r.template get<V>(M_SX + q);
+            }
             gl[0] = r.template get<V>(H_SX);
             gl[1] = r.template get<V>(H_SY);
             V gr[3][3];
@@ -751,11 +794,16 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
             const V j0 = mx.template get<V>(3), j1 = mx.template get<V>(4), j2 = mx.template get<V>(5);
             const V nB0 = -B0, nB1 = -B1, nB2 = -B2;
             const V jxB[3] = {vfma(j1, B2, j2 * nB1), vfma(j2, B0, j0 * nB2), vfma(j0, B1, j1 * nB0)};
-            rr[0] = r0;
+            if constexpr (UPWD)
+                rr[0] = r0 + upz[0];
+            else
+                rr[0] = r0;
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
                 const V pg = vfma(c.inv_cp, mx.template get<V>(q), gl[q]);
                 rr[1 + q]  = vfma(irho, jxB[q], vfma(ncs2, pg, t[q]));
+                if constexpr (UPWD)
+                    rr[1 + q] = rr[1 + q] + upz[1 + q];
             }
             val[0] = lnrho;
             val[1] = ux;
@@ -766,9 +814,9 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
             TWords<REC_MN> r;
             TWords<3> a;
             TWords<4> uw; /* lnrho, ux, uy, uz */
-            r.load(rec + 2 * M_SX);
+            r.load(rec + 2 * TM::HN);
             a.load(aslot);
-            uw.load(ch.tl + ZQ0 + (uint32_t)(p & 7) * ZQ_W);
+            uw.load(ch.tl + TM::ZQ0 + (uint32_t)(p & 7) * ZQ_W);
             const V ent = w[3].template get<V>(0);
             V gs[3], s2[4], dzAx, dzAy, unused;
             z_derivs(w, 0, c.d1[2], c.d2[2], gs[2], s2[0]);
@@ -853,7 +901,7 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
         }
         i0 += g.pxy;
         i1 += g.pxy;
-        rec = ++r5 == REC_SLOTS ? (r5 = 0, rec - (REC_SLOTS - 1) * REC_W) : rec + REC_W;
+        rec = ++r5 == REC_SLOTS ? (r5 = 0, rec - (REC_SLOTS - 1) * TM::REC_W) : rec + TM::REC_W;
     }
     return ok;
 }
@@ -870,7 +918,7 @@ loads_into(const int ring, const int sl, const int pfirst, const int plast, cons
     return n;
 }
 
-template <typename V, bool PREV>
+template <typename V, bool PREV, bool UPWD>
 __global__ void __launch_bounds__(THREADS, 1)
 solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
                    const FieldsT<typename Pack<V>::T> f, const __grid_constant__ SplitCoef<V> c,
@@ -937,12 +985,12 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
     T* prev = reinterpret_cast<T*>(smem_raw + S::P_OFF);
     if (role == 0) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_INPLANE));
-        ok = inplane_role<V, 0>(&maps, c, ch, smem, cell_off, ly == 0 && lx == 0, PREV, x0, y0,
+        ok = inplane_role<V, 0, UPWD>(&maps, c, ch, smem, cell_off, ly == 0 && lx == 0, PREV, x0, y0,
                                 skip_last);
     }
     else if (role == 1) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_INPLANE));
-        ok = inplane_role<V, 1>(&maps, c, ch, smem, cell_off, false, PREV, x0, y0, skip_last);
+        ok = inplane_role<V, 1, UPWD>(&maps, c, ch, smem, cell_off, false, PREV, x0, y0, skip_last);
     }
     else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_SOLVE));
@@ -953,7 +1001,7 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
                 rf.out[k]  = f.out[k];
                 rf.outl[k] = f.out_lo[k];
             }
-            ok = solve_role<V, 0, PREV>(g, rf, c, rk, ch, prev, lx, ly, x, y, false, cfl_sum, cs2,
+            ok = solve_role<V, 0, PREV, UPWD>(g, rf, c, rk, ch, prev, lx, ly, x, y, false, cfl_sum, cs2,
                                         cm);
         }
         else {
@@ -962,7 +1010,7 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
                 rf.out[k]  = f.out[4 + k];
                 rf.outl[k] = f.out_lo[4 + k];
             }
-            ok = solve_role<V, 1, PREV>(g, rf, c, rk, ch, prev, lx, ly, x, y, cfl != nullptr, cfl_sum,
+            ok = solve_role<V, 1, PREV, UPWD>(g, rf, c, rk, ch, prev, lx, ly, x, y, cfl != nullptr, cfl_sum,
                                         cs2, cm);
         }
     }
@@ -1031,39 +1079,42 @@ launch_split(const Geom& g, const SplitMaps& tm, const FieldsT<T>& f, const Sten
     r.beta = Pack<V>::dup(rk.beta);
     r.ab   = Pack<V>::dup(rk.ab);
     const bool sum = pc.cfl_sum != 0, skip = pc.debug_skip_load != 0;
-    if (rk.step > 0)
-        solve_split_kernel<V, true><<<bpg, tpb, S::SMEM_BYTES, stream>>>(
-            tm, g, f, c, r, pc.zlo, pc.zhi, zc, err, cfl, sum, (T)pc.cs2_sound, skip);
+    auto launch = [&](auto kernel) {
+        kernel<<<bpg, tpb, S::SMEM_BYTES, stream>>>(tm, g, f, c, r, pc.zlo, pc.zhi, zc, err, cfl, sum,
+                                                    (T)pc.cs2_sound, skip);
+    };
+    if (pc.upwind)
+        rk.step > 0 ? launch(solve_split_kernel<V, true, true>)
+                    : launch(solve_split_kernel<V, false, true>);
     else
-        solve_split_kernel<V, false><<<bpg, tpb, S::SMEM_BYTES, stream>>>(
-            tm, g, f, c, r, pc.zlo, pc.zhi, zc, err, cfl, sum, (T)pc.cs2_sound, skip);
+        rk.step > 0 ? launch(solve_split_kernel<V, true, false>)
+                    : launch(solve_split_kernel<V, false, false>);
     if (launches)
         ++*launches;
     return cudaGetLastError();
-}
-
-template <typename V, bool PREV>
-cudaError_t
-init_split_form()
-{
-    const void* fn = (const void*)solve_split_kernel<V, PREV>;
-    cudaFuncAttributes a;
-    const cudaError_t e = cudaFuncGetAttributes(&a, fn);
-    if (e != cudaSuccess)
-        return e;
-    /* setmaxnreg only moves registers that the block was launched with */
-    if (a.numRegs * ROLES < 2 * (REGS_INPLANE + REGS_SOLVE))
-        return cudaErrorInvalidConfiguration;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)SplitTile<V>::SMEM_BYTES);
 }
 
 template <typename V>
 cudaError_t
 init_split()
 {
-    const cudaError_t e = init_split_form<V, true>();
-    return e != cudaSuccess ? e : init_split_form<V, false>();
+    const void* forms[4] = {
+        (const void*)solve_split_kernel<V, false, false>, (const void*)solve_split_kernel<V, true, false>,
+        (const void*)solve_split_kernel<V, false, true>, (const void*)solve_split_kernel<V, true, true>};
+    for (const void* fn : forms) {
+        cudaFuncAttributes a;
+        cudaError_t e = cudaFuncGetAttributes(&a, fn);
+        if (e != cudaSuccess)
+            return e;
+        /* setmaxnreg only moves registers that the block was launched with */
+        if (a.numRegs * ROLES < 2 * (REGS_INPLANE + REGS_SOLVE))
+            return cudaErrorInvalidConfiguration;
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)SplitTile<V>::SMEM_BYTES);
+        if (e != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
 }
 
 } // namespace

@@ -44,6 +44,16 @@ def test_split_kernel_equals_plain(n, precision):
     np.testing.assert_allclose(ma, mb, rtol=1e-13 if precision == 0 else 6e-6)
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", [(34, 7, 5), (66, 16, 11), (150, 13, 17)])
+def test_split_kernel_equals_plain_with_upwinding(n, precision):
+    a, ma, _ = run(n, precision, 1, upwind=1)
+    b, mb, _ = run(n, precision, 0, upwind=1)
+    err = np.abs(a - b).reshape(8, -1).max(axis=1) / np.abs(a).reshape(8, -1).max(axis=1)
+    assert err.max() <= (1e-14 if precision == 0 else 6e-6), err
+    np.testing.assert_allclose(ma, mb, rtol=1e-13 if precision == 0 else 6e-6)
+
+
 def test_z_boxes_of_any_size_give_the_same_bits():
     """Chunks start and end anywhere: the planes of a substep solved in uneven z boxes."""
     n = (40, 12, 19)
