@@ -290,6 +290,7 @@ acDeviceCreate(const int id, const AcMeshInfo device_config, Device* device_hand
         }                                                                                     \
     } while (0)
 
+    d->used_streams = 1u; /* stream 0: the set-up below */
     for (int s = 0; s < NUM_STREAMS; ++s)
         CREATE_CHECK(cudaStreamCreateWithFlags(&d->streams[s], cudaStreamNonBlocking));
 
@@ -310,16 +311,18 @@ acDeviceCreate(const int id, const AcMeshInfo device_config, Device* device_hand
     for (int q = 0; q < AC_NF; ++q)
         d->in_idx[q] = 0;
 
-    /* small scratch block: [partials 2*blocks][result 2][counter, err] */
+    CREATE_CHECK(cudaMallocHost((void**)&d->host_result, 4 * sizeof(double)));
+    memset(d->host_result, 0, 4 * sizeof(double));
+    d->red.result  = d->host_result;
+    d->err_flag    = (int*)(d->host_result + 2);
+    /* small scratch block: [partials 2*blocks][counter, nonfinite][cfl] */
     const int blocks    = ac_reduce_blocks(d->geom);
     d->red.max_blocks   = blocks;
     const size_t rbytes = (2 * (size_t)blocks + 2) * sizeof(double) + 128;
     CREATE_CHECK(cudaMalloc((void**)&d->red.partials, rbytes));
     CREATE_CHECK(cudaMemsetAsync(d->red.partials, 0, rbytes, d->streams[0]));
-    d->red.result  = d->red.partials + 2 * (size_t)blocks;
-    d->red.nonfinite = (unsigned int*)(d->red.result + 1);
-    d->red.counter = (unsigned int*)(d->red.result + 2);
-    d->err_flag    = (int*)(d->red.counter + 4);
+    d->red.counter   = (unsigned int*)(d->red.partials + 2 * (size_t)blocks);
+    d->red.nonfinite = d->red.counter + 1;
     d->cfl         = (unsigned long long*)(d->red.counter + 8);
     d->tmap_ok     = ac_make_tensor_map(&d->tmap[0], d->hi[0], d->geom, precision) &&
                  ac_make_tensor_map(&d->tmap[1], d->hi[1], d->geom, precision);
@@ -329,7 +332,6 @@ acDeviceCreate(const int id, const AcMeshInfo device_config, Device* device_hand
                   ac_make_split_maps(&d->smaps[1], d->hi[1], d->lo[1], d->geom, precision);
     if (d->split_ok)
         CREATE_CHECK(ac_solve_split_init(precision));
-    CREATE_CHECK(cudaMallocHost((void**)&d->host_result, 2 * sizeof(double)));
     CREATE_CHECK(ensure_bfield(d));
     CREATE_CHECK(cudaStreamSynchronize(d->streams[0]));
 #undef CREATE_CHECK
@@ -364,18 +366,14 @@ acDevicePrintInfo(const Device d)
     return AC_SUCCESS;
 }
 
-/* Reads and clears the device error word (set by a kernel whose bounded wait
- * on an mbarrier gave up); nonzero means the last results are invalid. */
+/* Reads and clears the error word (set by a kernel whose bounded wait on an
+ * mbarrier gave up; page-locked, so a wait for the kernel's stream is enough);
+ * nonzero means the last results are invalid. */
 static AcResult
-check_device_error(const Device d, cudaStream_t st)
+check_device_error(const Device d)
 {
-    int err = 0;
-    AC_CUDA_CHECK(cudaMemcpyAsync(&err, d->err_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-    AC_CUDA_CHECK(cudaStreamSynchronize(st));
-    if (err) {
+    if (__atomic_exchange_n(d->err_flag, 0, __ATOMIC_RELAXED)) {
         fprintf(stderr, "astaroth_b200: a kernel timed out waiting for its TMA loads\n");
-        AC_CUDA_CHECK(cudaMemsetAsync(d->err_flag, 0, sizeof(int), st));
-        AC_CUDA_CHECK(cudaStreamSynchronize(st));
         return AC_FAILURE;
     }
     return AC_SUCCESS;
@@ -388,14 +386,13 @@ acDeviceSynchronizeStream(const Device d, const Stream stream)
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
     if (stream == STREAM_ALL) {
-        for (int s = 0; s < NUM_STREAMS; ++s)
-            AC_CUDA_CHECK(cudaStreamSynchronize(d->streams[s]));
-        return check_device_error(d, d->streams[0]);
+        AC_CUDA_CHECK(wait_used_streams(d));
+        return check_device_error(d);
     }
     if (!stream_ok(stream))
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaStreamSynchronize(d->streams[stream]));
-    return check_device_error(d, d->streams[stream]);
+    return check_device_error(d);
 }
 
 extern "C" AcResult
@@ -600,16 +597,16 @@ acDeviceLoadVertexBuffer(const Device d, const Stream stream, const AcMesh host_
     if (d->precision == 0) {
         AC_CUDA_CHECK(cudaMemcpyAsync(arr64(d, b, h), host_mesh.vertex_buffer[h],
                                       n * sizeof(double), cudaMemcpyHostToDevice,
-                                      d->streams[stream]));
+                                      use_stream(d, stream)));
     }
     else {
         /* through the staging field: double -> (hi, lo) on the device */
         AC_CUDA_CHECK(cudaMemcpyAsync(d->staging, host_mesh.vertex_buffer[h], n * sizeof(double),
-                                      cudaMemcpyHostToDevice, d->streams[stream]));
+                                      cudaMemcpyHostToDevice, use_stream(d, stream)));
         AC_CUDA_CHECK(ac_launch_split(d->geom, d->staging, arr_hi(d, b, h), arr_lo(d, b, h),
-                                      d->streams[stream], &d->launches));
+                                      use_stream(d, stream), &d->launches));
         /* the staging field is shared by all streams: finish before returning */
-        AC_CUDA_CHECK(cudaStreamSynchronize(d->streams[stream]));
+        AC_CUDA_CHECK(cudaStreamSynchronize(use_stream(d, stream)));
     }
     return AC_SUCCESS;
 }
@@ -641,16 +638,16 @@ acDeviceStoreVertexBuffer(const Device d, const Stream stream, const VertexBuffe
     if (d->precision == 0) {
         AC_CUDA_CHECK(cudaMemcpyAsync(host_mesh->vertex_buffer[h], arr64(d, b, h),
                                       n * sizeof(double), cudaMemcpyDeviceToHost,
-                                      d->streams[stream]));
+                                      use_stream(d, stream)));
     }
     else {
         AC_CUDA_CHECK(ac_launch_join(d->geom, arr_hi(d, b, h), arr_lo(d, b, h), d->staging,
-                                     d->streams[stream], &d->launches));
+                                     use_stream(d, stream), &d->launches));
         AC_CUDA_CHECK(cudaMemcpyAsync(host_mesh->vertex_buffer[h], d->staging, n * sizeof(double),
-                                      cudaMemcpyDeviceToHost, d->streams[stream]));
+                                      cudaMemcpyDeviceToHost, use_stream(d, stream)));
     }
     /* The host array is ready when the call returns. */
-    AC_CUDA_CHECK(cudaStreamSynchronize(d->streams[stream]));
+    AC_CUDA_CHECK(cudaStreamSynchronize(use_stream(d, stream)));
     return AC_SUCCESS;
 }
 
@@ -672,11 +669,11 @@ acDeviceSetVertexBuffer(const Device d, const Stream stream, const VertexBufferH
     AC_CUDA_CHECK(cudaSetDevice(d->id));
     const int b = d->in_idx[h];
     if (d->precision == 0)
-        AC_CUDA_CHECK(ac_launch_fill(arr64(d, b, h), d->geom.cells, value, d->streams[stream],
+        AC_CUDA_CHECK(ac_launch_fill(arr64(d, b, h), d->geom.cells, value, use_stream(d, stream),
                                      &d->launches));
     else
         AC_CUDA_CHECK(ac_launch_fill_comp(arr_hi(d, b, h), arr_lo(d, b, h), d->geom.cells, value,
-                                          d->streams[stream], &d->launches));
+                                          use_stream(d, stream), &d->launches));
     return AC_SUCCESS;
 }
 
@@ -703,7 +700,7 @@ acDeviceFlushOutputBuffers(const Device d, const Stream stream)
     if (!d || !stream_ok(stream))
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
-    return clear_buffers(d, d->streams[stream], false, true);
+    return clear_buffers(d, use_stream(d, stream), false, true);
 }
 
 extern "C" AcResult
@@ -712,7 +709,7 @@ acDeviceResetMesh(const Device d, const Stream stream)
     if (!d || !stream_ok(stream))
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
-    return clear_buffers(d, d->streams[stream], true, true);
+    return clear_buffers(d, use_stream(d, stream), true, true);
 }
 
 /* ---- integration ---- */
@@ -855,7 +852,7 @@ acDeviceIntegrateSubstep(const Device d, const Stream stream, const int step_num
         return AC_FAILURE;
     }
     AC_CUDA_CHECK(cudaSetDevice(d->id));
-    AC_CUDA_CHECK(launch_substep(d, d->streams[stream], step_number, dt, &d->launches,
+    AC_CUDA_CHECK(launch_substep(d, use_stream(d, stream), step_number, dt, &d->launches,
                                  (int)start.z - NGHOST, (int)end.z - NGHOST));
     if (step_number == 2)
         d->out_set = 0;
@@ -869,7 +866,7 @@ acDevicePeriodicBoundcondStep(const Device d, const Stream stream, const VertexB
     if (!d || !stream_ok(stream) || (int)h < 0 || h >= NUM_VTXBUF_HANDLES)
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
-    AC_CUDA_CHECK(launch_periodic(d, d->streams[stream], h, 1, start, end, &d->launches));
+    AC_CUDA_CHECK(launch_periodic(d, use_stream(d, stream), h, 1, start, end, &d->launches));
     return AC_SUCCESS;
 }
 
@@ -880,7 +877,7 @@ acDevicePeriodicBoundconds(const Device d, const Stream stream, const Volume sta
     if (!d || !stream_ok(stream))
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
-    AC_CUDA_CHECK(launch_periodic(d, d->streams[stream], 0, AC_NF, start, end, &d->launches));
+    AC_CUDA_CHECK(launch_periodic(d, use_stream(d, stream), 0, AC_NF, start, end, &d->launches));
     return AC_SUCCESS;
 }
 
@@ -907,7 +904,7 @@ acDeviceIntegrateStep(const Device d, const Stream stream, const AcReal dt)
     if (!d || !stream_ok(stream))
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
-    cudaStream_t st = d->streams[stream];
+    cudaStream_t st = use_stream(d, stream);
     /* All fields must be in the same buffer for the graph (true unless the
      * caller swapped single fields); otherwise run the launches directly. */
     const int parity = in_block_index(d);
@@ -973,9 +970,7 @@ reduce_common(const Device d, const Stream stream, const AcReduction r, const in
     AC_CUDA_CHECK(cudaSetDevice(d->id));
     /* Reductions observe all previously issued work of this device
      * (the reference synchronizes the device first, reductions.cu:103). */
-    for (int s = 0; s < NUM_STREAMS; ++s)
-        if (s != (int)stream)
-            AC_CUDA_CHECK(cudaStreamSynchronize(d->streams[s]));
+    AC_CUDA_CHECK(wait_used_streams(d, (int)stream));
     const void* fp[4];
     const float* lo[4] = {nullptr, nullptr, nullptr, nullptr};
     for (int q = 0; q < kind; ++q) {
@@ -988,13 +983,10 @@ reduce_common(const Device d, const Stream stream, const AcReduction r, const in
             lo[q] = arr_lo(d, b, h[q]);
         }
     }
-    cudaStream_t st = d->streams[stream];
-    AC_CUDA_CHECK(cudaMemsetAsync(d->red.nonfinite, 0, sizeof(unsigned int), st));
+    cudaStream_t st = use_stream(d, stream);
     AC_CUDA_CHECK(ac_launch_reduce(d->geom, fp, lo, kind, d->precision, map, r.reduce_op, d->red,
                                    st, &d->launches));
-    /* the result and the non-finite flag behind it */
-    AC_CUDA_CHECK(cudaMemcpyAsync(d->host_result, d->red.result, 2 * sizeof(double),
-                                  cudaMemcpyDeviceToHost, st));
+    /* the kernel writes the result and the non-finite flag to page-locked memory */
     AC_CUDA_CHECK(cudaStreamSynchronize(st));
     *result           = d->host_result[0];
     unsigned int flag = 0;
@@ -1124,10 +1116,10 @@ acDeviceCalcTimestep(const Device d, const Stream stream)
     const double cs2 = d->config.real_params[AC_cs_sound] * d->config.real_params[AC_cs_sound];
     if (d->precision == 0)
         AC_CUDA_CHECK(ac_launch_cfl<double>(d->geom, fields64(d), sc, cs2, d->cfl,
-                                            d->streams[stream], &d->launches));
+                                            use_stream(d, stream), &d->launches));
     else
         AC_CUDA_CHECK(ac_launch_cfl<float>(d->geom, fields32(d), sc, cs2, d->cfl,
-                                           d->streams[stream], &d->launches));
+                                           use_stream(d, stream), &d->launches));
     d->out_set = 0;
     return AC_SUCCESS;
 }
@@ -1163,9 +1155,8 @@ device_outputs(Device d, const cudaStream_t* st, double v[NUM_REAL_OUTPUTS])
             return e;
     }
     else {
-        for (int s = 0; s < NUM_STREAMS; ++s)
-            if ((e = cudaStreamSynchronize(d->streams[s])) != cudaSuccess)
-                return e;
+        if ((e = wait_used_streams(d)) != cudaSuccess)
+            return e;
     }
     unsigned long long w[3];
     if ((e = cudaMemcpy(w, d->cfl, sizeof(w), cudaMemcpyDeviceToHost)) != cudaSuccess)
@@ -1242,7 +1233,7 @@ acDeviceFinishReduceReal(Device d, const Stream stream, AcReal* result, const Ac
 {
     if (!d || !stream_ok(stream))
         return AC_FAILURE;
-    return finish_reduce(d, d->streams[stream], result, kernel, reduce_op, output);
+    return finish_reduce(d, use_stream(d, stream), result, kernel, reduce_op, output);
 }
 
 extern "C" AcResult
@@ -1281,7 +1272,7 @@ acDeviceGetStreamHandle(const Device d, const Stream stream)
 {
     if (!d || !stream_ok(stream))
         return NULL;
-    return (void*)d->streams[stream];
+    return (void*)use_stream(d, stream);
 }
 
 extern "C" unsigned long long

@@ -71,7 +71,7 @@ acDeviceLoadAdjoint(const Device d, const Stream stream, const AcReal* const* la
     AC_CUDA_CHECK(cudaSetDevice(d->id));
     if (ensure_adjoint(d) != AC_SUCCESS)
         return AC_FAILURE;
-    cudaStream_t st   = d->streams[stream];
+    cudaStream_t st   = use_stream(d, stream);
     const size_t cells = (size_t)adj_geom(d).cells;
     const size_t fb   = cells * sizeof(double);
     for (int q = 0; q < AC_NF; ++q) {
@@ -97,7 +97,7 @@ acDeviceStoreAdjoint(const Device d, const Stream stream, AcReal* const* lam_f)
     for (int q = 0; q < AC_NF; ++q)
         if (lam_f[q])
             AC_CUDA_CHECK(cudaMemcpyAsync(lam_f[q], d->adj_lf + (size_t)q * cells, fb,
-                                          cudaMemcpyDeviceToDevice, d->streams[stream]));
+                                          cudaMemcpyDeviceToDevice, use_stream(d, stream)));
     return AC_SUCCESS;
 }
 
@@ -145,7 +145,7 @@ acDeviceIntegrateSubstepAdjoint(const Device d, const Stream stream, const int s
         return AC_FAILURE;
     }
     AC_CUDA_CHECK(cudaSetDevice(d->id));
-    AC_CUDA_CHECK(launch_adjoint(d, d->streams[stream], step_number, dt, NULL));
+    AC_CUDA_CHECK(launch_adjoint(d, use_stream(d, stream), step_number, dt, NULL));
     return AC_SUCCESS;
 }
 
@@ -203,7 +203,7 @@ acDeviceAdjointTapeForward(const Device d, const Stream stream, const int steps,
                                                            sizeof(double)));
         d->adj_tape_states = 3 * steps;
     }
-    cudaStream_t st = d->streams[stream];
+    cudaStream_t st = use_stream(d, stream);
     /* the recompute is one CUDA graph per in-block, kept for the next call
      * with the same steps, dt and stream (one capture per checkpoint length) */
     if (!(d->tape_valid[blk] && d->tape_steps[blk] == steps && d->tape_dt[blk] == dt &&
@@ -251,7 +251,7 @@ acDeviceAdjointTapeBackward(const Device d, const Stream stream, const int steps
     if (ensure_adjoint(d) != AC_SUCCESS)
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
-    cudaStream_t st             = d->streams[stream];
+    cudaStream_t st             = use_stream(d, stream);
     const size_t state_elems    = (size_t)AC_NF * adj_geom(d).cells;
     for (int n = steps - 1; n >= 0; --n)
         for (int s = 2; s >= 0; --s)
@@ -266,8 +266,7 @@ acDeviceGetParamAdjoints(const Device d, AcReal* nu_bar, AcReal* eta_bar)
     if (!d || !nu_bar || !eta_bar || !d->adj_pgrad)
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
-    for (int s = 0; s < NUM_STREAMS; ++s)
-        AC_CUDA_CHECK(cudaStreamSynchronize(d->streams[s]));
+    AC_CUDA_CHECK(wait_used_streams(d));
     double v[2];
     AC_CUDA_CHECK(cudaMemcpy(v, d->adj_pgrad, sizeof(v), cudaMemcpyDeviceToHost));
     *nu_bar  = v[0];

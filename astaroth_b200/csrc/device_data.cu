@@ -75,7 +75,7 @@ acDeviceLoadVertexBufferWithOffset(const Device d, const Stream stream, const Ac
         return AC_SUCCESS;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
     const int b       = d->in_idx[h];
-    cudaStream_t st   = d->streams[stream];
+    cudaStream_t st   = use_stream(d, stream);
     const double* hp  = host_mesh.vertex_buffer[h] + s0;
     if (d->precision == 0) {
         AC_CUDA_CHECK(cudaMemcpyAsync(arr64(d, b, h) + d0, hp, n * sizeof(double),
@@ -122,7 +122,7 @@ acDeviceStoreVertexBufferWithOffset(const Device d, const Stream stream,
         return AC_SUCCESS;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
     const int b     = d->in_idx[h];
-    cudaStream_t st = d->streams[stream];
+    cudaStream_t st = use_stream(d, stream);
     double* hp      = host_mesh->vertex_buffer[h] + d0;
     if (d->precision == 0) {
         AC_CUDA_CHECK(cudaMemcpyAsync(hp, arr64(d, b, h) + s0, n * sizeof(double),
@@ -169,7 +169,7 @@ acDeviceTransferVertexBufferWithOffset(const Device from, const Stream stream,
     if (n == 0)
         return AC_SUCCESS;
     AC_CUDA_CHECK(cudaSetDevice(from->id));
-    cudaStream_t st = from->streams[stream];
+    cudaStream_t st = use_stream(from, stream);
     const int fb = from->in_idx[h], tb = to->in_idx[h];
     if (from->precision == 0) {
         AC_CUDA_CHECK(cudaMemcpyPeerAsync(arr64(to, tb, h) + d0, to->id, arr64(from, fb, h) + s0,
@@ -184,7 +184,7 @@ acDeviceTransferVertexBufferWithOffset(const Device from, const Stream stream,
                                       n * sizeof(double), st));
     AC_CUDA_CHECK(cudaStreamSynchronize(st));
     AC_CUDA_CHECK(cudaSetDevice(to->id));
-    cudaStream_t tst = to->streams[stream];
+    cudaStream_t tst = use_stream(to, stream);
     AC_CUDA_CHECK(ac_launch_split_range(to->geom, to->staging, arr_hi(to, tb, h),
                                         arr_lo(to, tb, h), d0, n, tst, &to->launches));
     AC_CUDA_CHECK(cudaStreamSynchronize(tst));
@@ -260,7 +260,7 @@ acDeviceVolumeCopy(const Device d, const Stream stream, const AcReal* in, const 
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
     AC_CUDA_CHECK(ac_launch_volume_copy(in, in_offset, in_volume, out, out_offset, out_volume, nn,
-                                        d->streams[stream], &d->launches));
+                                        use_stream(d, stream), &d->launches));
     return AC_SUCCESS;
 }
 
@@ -303,7 +303,7 @@ acDeviceLoadMeshStaged(const Device d, const Stream stream, const AcMesh host_me
     AC_CUDA_CHECK(cudaSetDevice(d->id));
     const bool first = d->stage == nullptr;
     AC_CUDA_CHECK(ensure_stage(d));
-    cudaStream_t st = d->streams[stream];
+    cudaStream_t st = use_stream(d, stream);
     if (!first) /* the previous commit has read the stage */
         AC_CUDA_CHECK(cudaStreamWaitEvent(st, d->stage_read, 0));
     const size_t n = (size_t)d->geom.mx * d->geom.my * d->geom.mz;
@@ -320,7 +320,7 @@ acDeviceCommitStagedMesh(const Device d, const Stream stream)
     if (!d || !stream_ok(stream) || !d->stage)
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
-    cudaStream_t st = d->streams[stream];
+    cudaStream_t st = use_stream(d, stream);
     AC_CUDA_CHECK(cudaStreamWaitEvent(st, d->stage_loaded, 0));
     const size_t n = (size_t)d->geom.mx * d->geom.my * d->geom.mz;
     for (int q = 0; q < AC_NF; ++q) {
@@ -351,10 +351,10 @@ acDeviceLoadMeshDevice(const Device d, const Stream stream, const AcReal* const*
         const int b = d->in_idx[q];
         if (d->precision == 0)
             AC_CUDA_CHECK(cudaMemcpyAsync(arr64(d, b, q), src[q], n * sizeof(double),
-                                          cudaMemcpyDeviceToDevice, d->streams[stream]));
+                                          cudaMemcpyDeviceToDevice, use_stream(d, stream)));
         else
             AC_CUDA_CHECK(ac_launch_split(d->geom, src[q], arr_hi(d, b, q), arr_lo(d, b, q),
-                                          d->streams[stream], &d->launches));
+                                          use_stream(d, stream), &d->launches));
     }
     return AC_SUCCESS;
 }
@@ -372,10 +372,10 @@ acDeviceStoreMeshDevice(const Device d, const Stream stream, AcReal* const* dst)
         const int b = d->in_idx[q];
         if (d->precision == 0)
             AC_CUDA_CHECK(cudaMemcpyAsync(dst[q], arr64(d, b, q), n * sizeof(double),
-                                          cudaMemcpyDeviceToDevice, d->streams[stream]));
+                                          cudaMemcpyDeviceToDevice, use_stream(d, stream)));
         else
             AC_CUDA_CHECK(ac_launch_join(d->geom, arr_hi(d, b, q), arr_lo(d, b, q), dst[q],
-                                         d->streams[stream], &d->launches));
+                                         use_stream(d, stream), &d->launches));
     }
     return AC_SUCCESS;
 }
@@ -432,7 +432,7 @@ copy_planes(const Device d, const Stream stream, const int z0, const int nplanes
     /* one launch for all arrays (the buffer holds array a at a * bytes) */
     AC_CUDA_CHECK(ac_launch_planes(arrays, plane_arrays(d), (long long)z0 * d->geom.pxy * es,
                                    (long long)nplanes * d->geom.pxy * es, buffer, pack,
-                                   d->streams[stream], &d->launches));
+                                   use_stream(d, stream), &d->launches));
     return AC_SUCCESS;
 }
 
@@ -483,7 +483,7 @@ copy_box(const Device d, const Stream stream, const int3 start, const int3 dims,
     void* arrays[2 * AC_NF];
     packing_arrays(d, arrays);
     AC_CUDA_CHECK(ac_launch_box(arrays, plane_arrays(d), elem_size(d), d->geom, start, dims,
-                                buffer, pack, d->streams[stream], &d->launches));
+                                buffer, pack, use_stream(d, stream), &d->launches));
     return AC_SUCCESS;
 }
 
@@ -609,7 +609,7 @@ acDeviceReadMeshFromDisk(const Device d, const char* dir, const char* label, con
         m.info            = d->config;
         m.vertex_buffer[q] = buf;
         res = acDeviceLoadVertexBuffer(d, STREAM_DEFAULT, m, (VertexBufferHandle)q);
-        if (res == AC_SUCCESS && cudaStreamSynchronize(d->streams[STREAM_DEFAULT]) != cudaSuccess)
+        if (res == AC_SUCCESS && cudaStreamSynchronize(use_stream(d, STREAM_DEFAULT)) != cudaSuccess)
             res = AC_FAILURE;
     }
     free(buf);
@@ -638,8 +638,8 @@ acDeviceStoreBfield(const Device d, const Stream stream, AcReal* bx, AcReal* by,
     AcReal* out[3]  = {bx, by, bz};
     for (int c = 0; c < 3; ++c)
         AC_CUDA_CHECK(cudaMemcpyAsync(out[c], d->bfield + c * nm, nm * sizeof(double),
-                                      cudaMemcpyDeviceToHost, d->streams[stream]));
-    AC_CUDA_CHECK(cudaStreamSynchronize(d->streams[stream]));
+                                      cudaMemcpyDeviceToHost, use_stream(d, stream)));
+    AC_CUDA_CHECK(cudaStreamSynchronize(use_stream(d, stream)));
     return AC_SUCCESS;
 }
 

@@ -78,6 +78,29 @@ stream_ok(const Stream s)
     return (int)s >= 0 && (int)s < NUM_STREAMS;
 }
 
+/* Stream s of the device for work to be put into it.  The streams that were
+ * ever used are remembered (a bit that is only ever set), so that a wait for all
+ * of the device's streams passes over the others: 32 idle streams cost 45 us. */
+static inline cudaStream_t
+use_stream(const Device d, const Stream s)
+{
+    __atomic_fetch_or(&d->used_streams, 1u << (int)s, __ATOMIC_RELAXED);
+    return d->streams[s];
+}
+
+static inline cudaError_t
+wait_used_streams(const Device d, const int except = -1)
+{
+    const unsigned used = __atomic_load_n(&d->used_streams, __ATOMIC_RELAXED);
+    for (int s = 0; s < NUM_STREAMS; ++s)
+        if (s != except && (used >> s & 1u)) {
+            const cudaError_t e = cudaStreamSynchronize(d->streams[s]);
+            if (e != cudaSuccess)
+                return e;
+        }
+    return cudaSuccess;
+}
+
 static inline bool
 host_matches(const Device d, const AcMeshInfo& host)
 {

@@ -127,9 +127,10 @@ typedef FieldsT<float> Fields32;
 struct ReduceScratch {
     double* partials;        /* 2 doubles per block */
     unsigned int* counter;   /* zero between calls */
-    double* result;          /* 1 double, then the non-finite flag (result + 1) */
-    unsigned int* nonfinite; /* the low word of result[1]: 1 when a mapped value was NaN or
-                              * infinite; cleared before each call (may be null) */
+    double* result;          /* 1 double and, with nonfinite, 1 word behind it that says
+                              * whether a mapped value was NaN or infinite (page-locked host
+                              * memory or device memory) */
+    unsigned int* nonfinite; /* device word that collects it, zero between calls (may be null) */
     int max_blocks;
 };
 
@@ -164,7 +165,7 @@ struct device_s {
     int split_ok;
     CUtensorMap tmap[2]; /* 4-D (x, y, z, field) maps of the value (hi) array of each block */
     int tmap_ok;
-    int* err_flag;       /* device word set by kernels whose bounded waits gave up */
+    int* err_flag;       /* word in host_result set by kernels whose bounded waits gave up */
     /* CFL maxima of the last substep 2 (bit patterns of non-negative doubles):
      * [0] max |u|, [1] max Alfven speed |B|/sqrt(rho), [2] max |u| + sqrt(cs^2 + vA^2) */
     unsigned long long* cfl;
@@ -173,12 +174,15 @@ struct device_s {
     Geom geom;
     int precision;       /* 0 FP64, 1 FP32 compensated */
     cudaStream_t streams[NUM_STREAMS];
+    unsigned used_streams; /* bit s: stream s may have work (use_stream) */
     void* hi[2];         /* double* (FP64) or float* (FP32) value arrays per block */
     float* lo[2];        /* FP32 compensation arrays per block (NULL for FP64) */
     double* staging;     /* FP32: one field of doubles for host transfers */
     int in_idx[AC_NF];
     ReduceScratch red;
-    double* host_result; /* pinned */
+    /* page-locked words that kernels write: [0] the result of a reduction, [1] its
+     * non-finite flag, [2] err_flag */
+    double* host_result;
     StepGraph graphs[NUM_STREAMS][2];
     int solve_variant;   /* 0 = plain, else the tiled kernel AC_SOLVE_TILED_* */
     int debug_skip_load; /* acDeviceDebugSkipPlaneLoad */

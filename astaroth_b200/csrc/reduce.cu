@@ -123,27 +123,41 @@ reduce_kernel(const Geom g, const R f, const int map, const int op,
     const bool is_sum  = op == AC_REDUCE_OP_SUM;
     const double ident = op == AC_REDUCE_OP_MAX ? -INFINITY : INFINITY;
 
+    /* A warp takes an x row at a time, U cells per lane with their loads in flight
+     * together: a row per block with one load per thread left the kernel waiting
+     * for memory (256^3, one field: 106 -> 36 us). */
+    constexpr int U = 4;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int WARPS = kTpb / 32;
     DD acc{0.0, 0.0};
-    double ext          = ident;
-    bool bad            = false;
+    double ext           = ident;
+    bool bad             = false;
     const long long rows = (long long)g.ny * g.nz;
-    for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
-        const int j          = (int)(r % g.ny);
+    for (long long r = (long long)blockIdx.x * WARPS + warp; r < rows;
+         r += (long long)gridDim.x * WARPS) {
         const int k          = (int)(r / g.ny);
+        const int j          = (int)(r - (long long)k * g.ny);
         const long long base = geom_idx(g, NGHOST, j + NGHOST, k + NGHOST);
-        for (int i = threadIdx.x; i < g.nx; i += kTpb) {
-            const double v = map_value(map, f, base + i);
-            bad |= !isfinite(v);
-            if (is_sum)
-                acc = dd_add(acc, v);
-            else
-                ext = combine(op, ext, v);
+        for (int i0 = lane; i0 < g.nx; i0 += 32 * U) {
+            double v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) /* past the row's end: its last cell, not used below */
+                v[u] = map_value(map, f, base + min(i0 + 32 * u, g.nx - 1));
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (i0 + 32 * u >= g.nx)
+                    continue;
+                bad |= !isfinite(v[u]);
+                if (is_sum)
+                    acc = dd_add(acc, v[u]);
+                else
+                    ext = combine(op, ext, v[u]);
+            }
         }
     }
     if (__syncthreads_or(bad) && nonfinite && threadIdx.x == 0)
         atomicOr(nonfinite, 1u);
     /* warp */
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         if (is_sum) {
@@ -216,6 +230,8 @@ reduce_kernel(const Geom g, const R f, const int map, const int op,
         }
         *result  = is_sum ? b.hi + b.lo : x;
         *counter = 0u;
+        if (nonfinite)
+            *reinterpret_cast<unsigned int*>(result + 1) = atomicExch(nonfinite, 0u);
     }
 }
 
@@ -225,8 +241,9 @@ int
 ac_reduce_blocks(const Geom& g)
 {
     const long long rows = (long long)g.ny * g.nz;
-    const long long cap  = 148LL * 8;
-    return (int)(rows < cap ? rows : cap);
+    const long long want = (rows + 7) / 8; /* a row per warp */
+    const long long cap  = (long long)AC_SMS * 8;
+    return (int)(want < cap ? want : cap);
 }
 
 cudaError_t

@@ -59,6 +59,7 @@
  * AC_FAILURE.
  */
 #include <cuda.h>
+#include <atomic>
 
 #include "internal.h"
 #include "mhd_rhs.cuh"
@@ -1018,7 +1019,7 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
     if (cfl)
         cfl_commit(cm, red, cfl);
     if (!ok)
-        atomicExch(err, 1);
+        *(volatile int*)err = 1; /* (may be host memory) */
     /* no copy into this block's shared memory is left in flight */
     if (tid == 0) {
         drain_ring(bars, S::RING, [&](const int sl) {
@@ -1134,10 +1135,22 @@ ac_make_split_maps(SplitBufferMaps* m, void* hi, float* lo, const Geom& g, const
            ac_encode_field_map(&m->tile_lo, lo, g, 1, F::PXW, F::TY);
 }
 
+/* Once per GPU and precision (function attributes are the GPU's). */
 cudaError_t
 ac_solve_split_init(const int precision)
 {
-    return precision == 0 ? init_split<double>() : init_split<F2>();
+    static std::atomic<unsigned long long> done[2]; /* bit: device id */
+    int id        = 0;
+    cudaError_t e = cudaGetDevice(&id);
+    if (e != cudaSuccess)
+        return e;
+    const unsigned long long bit = id < 64 ? 1ull << id : 0;
+    if (done[precision] & bit)
+        return cudaSuccess;
+    e = precision == 0 ? init_split<double>() : init_split<F2>();
+    if (e == cudaSuccess)
+        done[precision] |= bit;
+    return e;
 }
 
 cudaError_t

@@ -455,7 +455,7 @@ solve_tiled_kernel(const __grid_constant__ CUtensorMap tmap, const Geom g, const
     if (cfl)
         cfl_commit(cm, xh, cfl); /* the exchange area is free after the last barrier */
     if (!ok)
-        atomicExch(err, 1);
+        *(volatile int*)err = 1; /* (may be host memory) */
     if (tid == 0)
         drain_ring(bars, RING, [&](const int sl) { return loads_into(sl, pfirst, plast, skip_last); });
 }
