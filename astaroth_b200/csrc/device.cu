@@ -783,7 +783,8 @@ launch_substep(Device d, cudaStream_t st, const int step, const double dt,
         }
         cfl = d->cfl;
     }
-    const bool split = tiled && d->split_ok && d->solve_variant != AC_SOLVE_TILED_TAPS;
+    const bool split = d->solve_variant != 0 && d->split_ok && blk >= 0 &&
+                       d->solve_variant != AC_SOLVE_TILED_TAPS;
     cudaError_t e;
     if (d->precision == 0) {
         const Fields64 f = fields64(d);

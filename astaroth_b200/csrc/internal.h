@@ -155,6 +155,7 @@ struct StepGraph {
  * compensation words). */
 struct SplitBufferMaps {
     CUtensorMap plane, tile, tile_lo;
+    int threads_load; /* no maps: the kernel's threads load the planes */
 };
 
 /* The two buffers of every field: block b holds all 8 fields of buffer b

@@ -60,6 +60,8 @@
  */
 #include <cuda.h>
 #include <atomic>
+#include <type_traits>
+#include <vector>
 
 #include "internal.h"
 #include "mhd_rhs.cuh"
@@ -74,7 +76,8 @@ using namespace tma_ring;
 constexpr int TX      = 32;
 constexpr int WARPS_Y = 4;                     /* warps per role */
 constexpr int ROLES   = 4;
-constexpr int THREADS = ROLES * WARPS_Y * TX;
+constexpr int STH     = WARPS_Y * TX; /* threads of a role */
+constexpr int THREADS = ROLES * STH;
 /* registers per thread: the block is launched with 128 each, and the in-plane
  * roles pass 8 to the solve roles (setmaxnreg; checked in init_split).  Measured
  * at 256^3, per step: FP64 3.01 ms against 3.26 with 128 each and 3.27 with 112
@@ -606,16 +609,23 @@ struct RoleFields {
  * previous-state slot. */
 template <bool PREV>
 __device__ __forceinline__ void
+update_store(const RoleFields<double>& f, const int k, const long long i0, const bool a0,
+             const double val, const double prev, const double rate, const RkV<double>& rk)
+{
+    double upd = rk.dt * rate;
+    if (PREV)
+        upd = fma(rk.ab, val - prev, upd);
+    const double o = fma(rk.beta, upd, val);
+    if (a0)
+        f.out[k][i0] = o;
+}
+template <bool PREV>
+__device__ __forceinline__ void
 update_store(const RoleFields<double>& f, const int k, const long long i0, const long long,
              const bool a0, const bool, const double val, const double* p, const double rate,
              const RkV<double>& rk)
 {
-    double upd = rk.dt * rate;
-    if (PREV)
-        upd = fma(rk.ab, val - p[k * SplitTile<double>::PFLD], upd);
-    const double o = fma(rk.beta, upd, val);
-    if (a0)
-        f.out[k][i0] = o;
+    update_store<PREV>(f, k, i0, a0, val, PREV ? p[k * SplitTile<double>::PFLD] : 0.0, rate, rk);
 }
 template <bool PREV>
 __device__ __forceinline__ void
@@ -669,21 +679,76 @@ cfl_cells(const F2 u2, const F2 b2, const F2 irho, const float cs2, float m[3], 
         cfl_accumulate(hi_of(u2), hi_of(b2), hi_of(irho), cs2, m, with_sum);
 }
 
-template <typename V, int GROUP, bool PREV, bool UPWD>
+/* Planes loaded by the threads of the solve roles, for FP64 meshes whose rows are
+ * no multiple of 16 bytes (nx odd), which TMA does not take: 8-byte asynchronous
+ * copies, whose completion arrives on the slot's mbarrier as TMA's does. */
+struct PlaneCopier {
+    static constexpr int N = 2; /* elements of a field's plane per thread */
+    typedef SplitTile<double> S;
+    static_assert(S::PLANE <= N * 2 * STH, "a field's plane");
+    int src[N]; /* offset in the plane, -1: none */
+    int t;
+    __device__ __forceinline__ void init(const Geom& g, const int t0, const int x0, const int y0)
+    {
+        t = t0;
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const int e = t + n * 2 * STH;
+            const int y = y0 + e / S::HXP, x = x0 + e % S::HXP;
+            src[n] = e < S::PLANE && x < g.mx && y < g.my ? x + y * g.px : -1;
+        }
+    }
+    /* plane L (interior z index) of all fields into slot sl; every thread of the
+     * two roles calls it */
+    __device__ __forceinline__ void copy(const Geom& g, const FieldsT<double>& f, const int L,
+                                         double* smem, const int sl, uint64_t* bar) const
+    {
+        const long long off = (long long)(L + NGHOST) * g.pxy;
+#pragma unroll
+        for (int q = 0; q < AC_NF; ++q)
+#pragma unroll
+            for (int n = 0; n < N; ++n)
+                if (src[n] >= 0)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                                     smem_addr(smem + sl * S::SLOT + q * S::PLANE + t + n * 2 * STH)),
+                                 "l"(f.in[q] + off + src[n])
+                                 : "memory");
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar))
+                     : "memory");
+    }
+};
+
+template <typename V, int GROUP, bool PREV, bool UPWD, bool LDG>
 __device__ __forceinline__ bool
 solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitCoef<V>& c,
            const RkV<V>& rk, const Chunk& ch, const typename Pack<V>::T* prev, const int lx,
            const int ly, const int x, const int y, const bool do_cfl,
-           const bool cfl_sum, const typename Pack<V>::T cs2, typename Pack<V>::T cm[3])
+           const bool cfl_sum, const typename Pack<V>::T cs2, typename Pack<V>::T cm[3],
+           const FieldsT<typename Pack<V>::T>& fields, typename Pack<V>::T* smem,
+           const bool skip_last)
 {
     typedef SplitTile<V> S;
     bool ok = true;
+    [[maybe_unused]] PlaneCopier pc;
+    /* plane L into its slot, if the chunk has it */
+    auto copy_plane = [&](const int L) {
+        if constexpr (LDG)
+            if (L <= ch.plast && !(skip_last && L == ch.plast)) {
+                const int sl = (L - ch.pfirst) % S::RING;
+                pc.copy(g, fields, L, smem, sl, &ch.rfull[sl]);
+            }
+    };
+    if constexpr (LDG) {
+        pc.init(g, (GROUP * WARPS_Y + ly) * TX + lx, x - lx, y - ly);
+        for (int i = 0; i < S::RING; ++i)
+            copy_plane(ch.pfirst + i);
+    }
     /* the stores of cells outside the mesh are skipped */
     const int y1  = y + WARPS_Y;
     const bool a0 = x < g.nx && y < g.ny, a1 = x < g.nx && y1 < g.ny;
     long long i0 = geom_idx(g, x + NGHOST, y + NGHOST, ch.z0 + NGHOST);
     long long i1 = geom_idx(g, x + NGHOST, y1 + NGHOST, ch.z0 + NGHOST);
-    constexpr bool WAITS = PREV || Pack<V>::N == 2; /* previous-state slots are used */
+    constexpr bool WAITS = !LDG && (PREV || Pack<V>::N == 2); /* previous-state slots are used */
     const typename Pack<V>::T* pcell =
         prev + 4 * GROUP * S::PFLD + ly * S::PXW + lx + (NGHOST - S::PX0);
     int pslot       = 0;
@@ -693,10 +758,19 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
     uint32_t r5 = 3 % REC_SLOTS; /* record slot of plane z0 = pfirst + 3 */
     uint32_t rec = ch.tl + r5 * TM::REC_W;
 #pragma unroll 1
-    for (int i = 0; i < 7; ++i)
+    for (int i = 0; i < 7; ++i) {
         interval_end();
+        copy_plane(ch.pfirst + i + S::RING);
+    }
 #pragma unroll 1
     for (int p = ch.z0; p < ch.z1; ++p) {
+        [[maybe_unused]] typename Pack<V>::T own[4] = {0, 0, 0, 0};
+        if constexpr (LDG && PREV)
+            if (a0) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    own[k] = f.out[k][i0];
+            }
         TWords<4> w[7];
 #pragma unroll
         for (int k = 0; k < 7; ++k)
@@ -770,6 +844,7 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
                 xw.store(xslot);
             }
             interval_end();
+            copy_plane(p + 4 + S::RING);
             if (WAITS && ok)
                 ok = mbar_wait_bounded(&ch.pfull[pslot], pphase);
             __syncwarp();
@@ -860,6 +935,7 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
                 xw.store(xslot + 2 * HX_N);
             }
             interval_end();
+            copy_plane(p + 4 + S::RING);
             if (WAITS && ok)
                 ok = mbar_wait_bounded(&ch.pfull[pslot], pphase);
             __syncwarp();
@@ -892,10 +968,14 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
             rr[3] = vfma(inv_T, H, vfma(c.K * irho, heat, adv));
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            update_store<PREV>(f, k, i0, i1, a0, a1, val[k],
-                               pcell + pslot * (S::PSLOT_BYTES / sizeof(typename Pack<V>::T)),
-                               rr[k], rk);
+        for (int k = 0; k < 4; ++k) {
+            if constexpr (LDG)
+                update_store<PREV>(f, k, i0, a0, val[k], own[k], rr[k], rk);
+            else
+                update_store<PREV>(f, k, i0, i1, a0, a1, val[k],
+                                   pcell + pslot * (S::PSLOT_BYTES / sizeof(typename Pack<V>::T)),
+                                   rr[k], rk);
+        }
         if (WAITS && ++pslot == S::PRING) {
             pslot = 0;
             pphase ^= 1;
@@ -904,6 +984,8 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
         i1 += g.pxy;
         rec = ++r5 == REC_SLOTS ? (r5 = 0, rec - (REC_SLOTS - 1) * TM::REC_W) : rec + TM::REC_W;
     }
+    if constexpr (LDG) /* no copy into this block's shared memory is left in flight */
+        asm volatile("cp.async.wait_all;" ::: "memory");
     return ok;
 }
 
@@ -919,7 +1001,8 @@ loads_into(const int ring, const int sl, const int pfirst, const int plast, cons
     return n;
 }
 
-template <typename V, bool PREV, bool UPWD>
+/* LDG: the planes by PlaneCopier instead of TMA */
+template <typename V, bool PREV, bool UPWD, bool LDG>
 __global__ void __launch_bounds__(THREADS, 1)
 solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
                    const FieldsT<typename Pack<V>::T> f, const __grid_constant__ SplitCoef<V> c,
@@ -951,7 +1034,7 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
 
     if (tid == 0) {
         for (int s = 0; s < S::NBARS; ++s)
-            mbar_init(&bars[s], 1);
+            mbar_init(&bars[s], LDG && s < S::RING ? 2 * STH : 1);
         fence_barrier_init();
     }
     __syncwarp();
@@ -964,7 +1047,7 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
     ch.tl                = tmem::lane_base(tbase, warp);
     ch.rfull             = bars;
     ch.pfull             = bars + S::RING;
-    if (tid == 0) {
+    if (!LDG && tid == 0) {
         const int pend = min(ch.plast, ch.pfirst + S::RING - 1);
         for (int q = ch.pfirst; q <= pend; ++q) {
             /* the fault-path test switch skips the load of the last plane */
@@ -986,7 +1069,7 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
     T* prev = reinterpret_cast<T*>(smem_raw + S::P_OFF);
     if (role == 0) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_INPLANE));
-        ok = inplane_role<V, 0, UPWD>(&maps, c, ch, smem, cell_off, ly == 0 && lx == 0, PREV, x0, y0,
+        ok = inplane_role<V, 0, UPWD>(&maps, c, ch, smem, cell_off, !LDG && ly == 0 && lx == 0, PREV, x0, y0,
                                 skip_last);
     }
     else if (role == 1) {
@@ -1002,8 +1085,8 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
                 rf.out[k]  = f.out[k];
                 rf.outl[k] = f.out_lo[k];
             }
-            ok = solve_role<V, 0, PREV, UPWD>(g, rf, c, rk, ch, prev, lx, ly, x, y, false, cfl_sum, cs2,
-                                        cm);
+            ok = solve_role<V, 0, PREV, UPWD, LDG>(g, rf, c, rk, ch, prev, lx, ly, x, y, false, cfl_sum, cs2,
+                                        cm, f, smem, skip_last);
         }
         else {
 #pragma unroll
@@ -1011,8 +1094,8 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
                 rf.out[k]  = f.out[4 + k];
                 rf.outl[k] = f.out_lo[4 + k];
             }
-            ok = solve_role<V, 1, PREV, UPWD>(g, rf, c, rk, ch, prev, lx, ly, x, y, cfl != nullptr, cfl_sum,
-                                        cs2, cm);
+            ok = solve_role<V, 1, PREV, UPWD, LDG>(g, rf, c, rk, ch, prev, lx, ly, x, y, cfl != nullptr, cfl_sum,
+                                        cs2, cm, f, smem, skip_last);
         }
     }
     __syncthreads();
@@ -1021,7 +1104,7 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
     if (!ok)
         *(volatile int*)err = 1; /* (may be host memory) */
     /* no copy into this block's shared memory is left in flight */
-    if (tid == 0) {
+    if (!LDG && tid == 0) {
         drain_ring(bars, S::RING, [&](const int sl) {
             return loads_into(S::RING, sl, ch.pfirst, ch.plast, skip_last);
         });
@@ -1064,7 +1147,8 @@ template <typename V, typename T>
 cudaError_t
 launch_split(const Geom& g, const SplitMaps& tm, const FieldsT<T>& f, const StencilCoef& sc,
              const PhysConst& pc, const RkCoef& rk, int* err, unsigned long long* cfl,
-             cudaStream_t stream, unsigned long long* launches, const int sms)
+             cudaStream_t stream, unsigned long long* launches, const int sms,
+             [[maybe_unused]] const bool threads_load)
 {
     typedef SplitTile<V> S;
     const int nzr = pc.zhi - pc.zlo;
@@ -1084,12 +1168,23 @@ launch_split(const Geom& g, const SplitMaps& tm, const FieldsT<T>& f, const Sten
         kernel<<<bpg, tpb, S::SMEM_BYTES, stream>>>(tm, g, f, c, r, pc.zlo, pc.zhi, zc, err, cfl, sum,
                                                     (T)pc.cs2_sound, skip);
     };
-    if (pc.upwind)
-        rk.step > 0 ? launch(solve_split_kernel<V, true, true>)
-                    : launch(solve_split_kernel<V, false, true>);
+    auto pick = [&](auto ldg) {
+        constexpr bool LDG = decltype(ldg)::value;
+        if (pc.upwind)
+            rk.step > 0 ? launch(solve_split_kernel<V, true, true, LDG>)
+                        : launch(solve_split_kernel<V, false, true, LDG>);
+        else
+            rk.step > 0 ? launch(solve_split_kernel<V, true, false, LDG>)
+                        : launch(solve_split_kernel<V, false, false, LDG>);
+    };
+    if constexpr (sizeof(T) == 8) {
+        if (threads_load)
+            pick(std::true_type{});
+        else
+            pick(std::false_type{});
+    }
     else
-        rk.step > 0 ? launch(solve_split_kernel<V, true, false>)
-                    : launch(solve_split_kernel<V, false, false>);
+        pick(std::false_type{});
     if (launches)
         ++*launches;
     return cudaGetLastError();
@@ -1099,9 +1194,15 @@ template <typename V>
 cudaError_t
 init_split()
 {
-    const void* forms[4] = {
-        (const void*)solve_split_kernel<V, false, false>, (const void*)solve_split_kernel<V, true, false>,
-        (const void*)solve_split_kernel<V, false, true>, (const void*)solve_split_kernel<V, true, true>};
+    std::vector<const void*> forms = {(const void*)solve_split_kernel<V, false, false, false>,
+                                      (const void*)solve_split_kernel<V, true, false, false>,
+                                      (const void*)solve_split_kernel<V, false, true, false>,
+                                      (const void*)solve_split_kernel<V, true, true, false>};
+    if constexpr (Pack<V>::N == 1)
+        forms.insert(forms.end(), {(const void*)solve_split_kernel<V, false, false, true>,
+                                   (const void*)solve_split_kernel<V, true, false, true>,
+                                   (const void*)solve_split_kernel<V, false, true, true>,
+                                   (const void*)solve_split_kernel<V, true, true, true>});
     for (const void* fn : forms) {
         cudaFuncAttributes a;
         cudaError_t e = cudaFuncGetAttributes(&a, fn);
@@ -1125,6 +1226,12 @@ ac_make_split_maps(SplitBufferMaps* m, void* hi, float* lo, const Geom& g, const
 {
     typedef SplitTile<double> D;
     typedef SplitTile<F2> F;
+    /* FP64 rows of an odd number of values are no multiple of 16 bytes: no tensor
+     * map, the threads load the planes.  125^3: 0.56 ms per step, the plain kernel
+     * 0.90 (128^3 by TMA 0.46). */
+    m->threads_load = precision == 0 && (g.nx & 1) && g.nx >= TX && g.ny >= WARPS_Y;
+    if (m->threads_load)
+        return true;
     if (!ac_tiled_supported(g, precision) || g.my < (precision == 0 ? D::HY : F::HY))
         return false;
     if (precision == 0)
@@ -1160,7 +1267,7 @@ ac_launch_solve_split64(const Geom& g, const SplitBufferMaps& in, const SplitBuf
                         const int sms)
 {
     return launch_split<double>(g, SplitMaps{in.plane, out.tile, out.tile_lo, in.tile_lo}, f, sc, pc,
-                                rk, err, cfl, stream, launches, sms);
+                                rk, err, cfl, stream, launches, sms, in.threads_load);
 }
 
 cudaError_t
@@ -1170,5 +1277,5 @@ ac_launch_solve_split32(const Geom& g, const SplitBufferMaps& in, const SplitBuf
                         const int sms)
 {
     return launch_split<F2>(g, SplitMaps{in.plane, out.tile, out.tile_lo, in.tile_lo}, f, sc, pc,
-                                rk, err, cfl, stream, launches, sms);
+                                rk, err, cfl, stream, launches, sms, in.threads_load);
 }

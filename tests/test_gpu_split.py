@@ -18,7 +18,7 @@ from astaroth_b200.device import CONFIG_PARAMS, Device, make_info, seeded_mesh
 pytestmark = pytest.mark.gpu
 
 AMP = dict(amp_scalar=1e-2, sigma_uu=3e-2, sigma_aa=3e-3)
-SIZES = [(32, 4, 3), (32, 8, 8), (34, 7, 5), (62, 9, 4), (66, 16, 11), (96, 12, 37), (150, 13, 17)]
+SIZES = [(33, 4, 3), (35, 9, 7), (63, 8, 12), (125, 13, 9), (32, 4, 3), (32, 8, 8), (34, 7, 5), (62, 9, 4), (66, 16, 11), (96, 12, 37), (150, 13, 17)]
 
 
 def run(n, precision, kernel, **params):
@@ -45,7 +45,7 @@ def test_split_kernel_equals_plain(n, precision):
 
 
 @pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("n", [(34, 7, 5), (66, 16, 11), (150, 13, 17)])
+@pytest.mark.parametrize("n", [(65, 6, 5), (34, 7, 5), (66, 16, 11), (150, 13, 17)])
 def test_split_kernel_equals_plain_with_upwinding(n, precision):
     a, ma, _ = run(n, precision, 1, upwind=1)
     b, mb, _ = run(n, precision, 0, upwind=1)
