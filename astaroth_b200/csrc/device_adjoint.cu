@@ -41,6 +41,14 @@ join_state(const Device d, cudaStream_t st, double* dst, unsigned long long* lau
     return cudaSuccess;
 }
 
+/* values of one slot array: the interior cells, an even number of them */
+static size_t
+adj_mu_stride(const Device d)
+{
+    const size_t n = (size_t)d->geom.nx * d->geom.ny * d->geom.nz;
+    return (n + 1) / 2 * 2;
+}
+
 static AcResult
 ensure_adjoint(const Device d)
 {
@@ -55,9 +63,10 @@ ensure_adjoint(const Device d)
     const size_t fb = (size_t)adj_geom(d).cells * sizeof(double);
     AC_CUDA_CHECK(cudaMalloc((void**)&d->adj_lf, AC_NF * fb));
     AC_CUDA_CHECK(cudaMalloc((void**)&d->adj_lw, AC_NF * fb));
-    AC_CUDA_CHECK(cudaMalloc((void**)&d->adj_mu, AC_MU_COUNT * fb));
+    const size_t mb = AC_MU_COUNT * adj_mu_stride(d) * sizeof(double);
+    AC_CUDA_CHECK(cudaMalloc((void**)&d->adj_mu, mb));
     AC_CUDA_CHECK(cudaMalloc((void**)&d->adj_pgrad, 2 * sizeof(double)));
-    AC_CUDA_CHECK(cudaMemset(d->adj_mu, 0, AC_MU_COUNT * fb));
+    AC_CUDA_CHECK(cudaMemset(d->adj_mu, 0, mb));
     if (d->precision != 0) /* the joined in-buffers of a per-substep adjoint call */
         AC_CUDA_CHECK(cudaMalloc((void**)&d->adj_state, AC_NF * fb));
     return AC_SUCCESS;
@@ -125,7 +134,7 @@ launch_adjoint(const Device d, cudaStream_t st, const int step, const double dt,
         a.lw[q] = d->adj_lw + (size_t)q * g.cells;
     }
     for (int m = 0; m < AC_MU_COUNT; ++m)
-        a.mu[m] = d->adj_mu + (size_t)m * g.cells;
+        a.mu[m] = d->adj_mu + (size_t)m * adj_mu_stride(d);
     const double alpha[3] = {0.0, -5.0 / 9.0, -153.0 / 128.0};
     const double beta[3]  = {1.0 / 3.0, 15.0 / 16.0, 8.0 / 15.0};
     return ac_launch_adjoint_substep(g, a, sc, pc, alpha[step], beta[step], dt, d->adj_pgrad,
