@@ -64,6 +64,8 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 periodic_rows_kernel(const Geom g, const ArrayList<T> fl, const int blocks_rows)
 {
+    ac_let_successor_start();
+    ac_wait_predecessor();
     T* a         = fl.p[blockIdx.y];
     const int nx = g.nx, ny = g.ny, nz = g.nz, mx = g.mx, my = g.my;
     constexpr int W = 16 / (int)sizeof(T); /* elements per 16-byte vector */
@@ -382,7 +384,7 @@ grid_for(const long long work, const int tpb)
 template <typename T>
 cudaError_t
 ac_launch_periodic(const Geom& g, T* const* arrays, const int n, const Volume start,
-                   const Volume end, cudaStream_t stream, unsigned long long* launches)
+                   const Volume end, cudaStream_t stream, unsigned long long* launches, const bool overlap)
 {
     if (n <= 0 || n > kMaxArrays)
         return cudaErrorInvalidValue;
@@ -407,12 +409,14 @@ ac_launch_periodic(const Geom& g, T* const* arrays, const int n, const Volume st
         bool vec = ((long long)g.px * (long long)sizeof(T)) % 16 == 0;
         for (int q = 0; q < n; ++q)
             vec = vec && ((uintptr_t)arrays[q] & 15) == 0;
-        if (vec)
-            periodic_rows_kernel<T, true><<<dim3((unsigned)(b_rows + b_cells), (unsigned)n), 256,
-                                            0, stream>>>(g, fl, (int)b_rows);
-        else
-            periodic_rows_kernel<T, false><<<dim3((unsigned)(b_rows + b_cells), (unsigned)n), 256,
-                                             0, stream>>>(g, fl, (int)b_rows);
+        const dim3 bpg((unsigned)(b_rows + b_cells), (unsigned)n);
+        const cudaError_t e =
+            vec ? ac_launch_overlapped(periodic_rows_kernel<T, true>, bpg, 256, 0, stream, overlap, g,
+                                       fl, (int)b_rows)
+                : ac_launch_overlapped(periodic_rows_kernel<T, false>, bpg, 256, 0, stream, overlap, g,
+                                       fl, (int)b_rows);
+        if (e != cudaSuccess)
+            return e;
     }
     else {
         const int3 s = make_int3((int)start.x, (int)start.y, (int)start.z);
@@ -429,10 +433,10 @@ ac_launch_periodic(const Geom& g, T* const* arrays, const int n, const Volume st
 
 template cudaError_t ac_launch_periodic<double>(const Geom&, double* const*, const int,
                                                 const Volume, const Volume, cudaStream_t,
-                                                unsigned long long*);
+                                                unsigned long long*, const bool);
 template cudaError_t ac_launch_periodic<float>(const Geom&, float* const*, const int,
                                                const Volume, const Volume, cudaStream_t,
-                                               unsigned long long*);
+                                               unsigned long long*, const bool);
 
 cudaError_t
 ac_launch_fill(double* ptr, const long long count, const double value, cudaStream_t stream,

@@ -731,7 +731,7 @@ ac_rk_coef(const int step, const double dt)
 
 cudaError_t
 launch_substep(Device d, cudaStream_t st, const int step, const double dt,
-               unsigned long long* launches, const int zlo, const int zhi)
+               unsigned long long* launches, const int zlo, const int zhi, const bool overlap)
 {
     if (fault_at("launch"))
         return cudaErrorLaunchFailure;
@@ -776,7 +776,7 @@ launch_substep(Device d, cudaStream_t st, const int step, const double dt,
      * reference's calc_timestep inside the third substep (mhdsolver.ac:611) */
     unsigned long long* cfl = nullptr;
     if (step == 2) {
-        if (first_box) {
+        if (first_box && !overlap) {
             const cudaError_t e = cudaMemsetAsync(d->cfl, 0, 3 * sizeof(unsigned long long), st);
             if (e != cudaSuccess)
                 return e;
@@ -789,7 +789,7 @@ launch_substep(Device d, cudaStream_t st, const int step, const double dt,
     if (d->precision == 0) {
         const Fields64 f = fields64(d);
         e = split   ? ac_launch_solve_split64(d->geom, d->smaps[blk], d->smaps[1 - blk], f, sc, pc, rk,
-                                              d->err_flag, cfl, st, launches)
+                                              d->err_flag, cfl, st, launches, AC_SMS, overlap)
             : tiled ? ac_launch_solve_tiled64(d->geom, &d->tmap[blk], f, sc, pc, rk, d->err_flag,
                                               cfl, st, launches)
                     : ac_launch_solve_plain64(d->geom, f, sc, pc, rk, cfl, st, launches);
@@ -797,7 +797,7 @@ launch_substep(Device d, cudaStream_t st, const int step, const double dt,
     else {
         const Fields32 f = fields32(d);
         e = split   ? ac_launch_solve_split32(d->geom, d->smaps[blk], d->smaps[1 - blk], f, sc, pc, rk,
-                                              d->err_flag, cfl, st, launches)
+                                              d->err_flag, cfl, st, launches, AC_SMS, overlap)
             : tiled ? ac_launch_solve_tiled32(d->geom, &d->tmap[blk], f, sc, pc, rk, d->err_flag,
                                               cfl, st, launches)
                     : ac_launch_solve_plain32(d->geom, f, sc, pc, rk, cfl, st, launches);
@@ -818,20 +818,20 @@ launch_substep(Device d, cudaStream_t st, const int step, const double dt,
 /* Periodic halo fill of the in-buffer of fields [q0, q0 + nq). */
 cudaError_t
 launch_periodic(Device d, cudaStream_t st, const int q0, const int nq, const Volume start,
-                const Volume end, unsigned long long* launches)
+                const Volume end, unsigned long long* launches, const bool overlap)
 {
     if (d->precision == 0) {
         double* a[AC_NF];
         for (int k = 0; k < nq; ++k)
             a[k] = arr64(d, d->in_idx[q0 + k], q0 + k);
-        return ac_launch_periodic<double>(d->geom, a, nq, start, end, st, launches);
+        return ac_launch_periodic<double>(d->geom, a, nq, start, end, st, launches, overlap);
     }
     float* a[2 * AC_NF];
     for (int k = 0; k < nq; ++k) {
         a[2 * k]     = arr_hi(d, d->in_idx[q0 + k], q0 + k);
         a[2 * k + 1] = arr_lo(d, d->in_idx[q0 + k], q0 + k);
     }
-    return ac_launch_periodic<float>(d->geom, a, 2 * nq, start, end, st, launches);
+    return ac_launch_periodic<float>(d->geom, a, 2 * nq, start, end, st, launches, overlap);
 }
 
 extern "C" AcResult
@@ -887,11 +887,17 @@ record_step(Device d, cudaStream_t st, const double dt, unsigned long long* laun
 {
     const Volume m0 = {0, 0, 0};
     const Volume m1 = {(size_t)d->geom.mx, (size_t)d->geom.my, (size_t)d->geom.mz};
+    /* the CFL words of substep 2 are cleared before the first kernel, so that each
+     * launch after it follows a kernel and can be set up while that one ends (six
+     * launches: 32^3 FP64 43.6 -> 41.9 us per step, 96 x 50 x 33 FP32 87 -> 75) */
+    cudaError_t e = cudaMemsetAsync(d->cfl, 0, 3 * sizeof(unsigned long long), st);
+    if (e != cudaSuccess)
+        return e;
     for (int s = 0; s < 3; ++s) {
-        cudaError_t e = launch_periodic(d, st, 0, AC_NF, m0, m1, launches);
+        e = launch_periodic(d, st, 0, AC_NF, m0, m1, launches, s > 0);
         if (e != cudaSuccess)
             return e;
-        e = launch_substep(d, st, s, dt, launches);
+        e = launch_substep(d, st, s, dt, launches, 0, -1, true);
         if (e != cudaSuccess)
             return e;
         acDeviceSwapBuffers(d);

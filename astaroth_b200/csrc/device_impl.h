@@ -138,9 +138,13 @@ is_z_box(const Device d, const Volume start, const Volume end)
            end.z <= (size_t)(d->geom.nz + NGHOST);
 }
 
-/* device.cu; [zlo, zhi) are the interior z planes solved (zhi < 0: all) */
+/* device.cu; [zlo, zhi) are the interior z planes solved (zhi < 0: all); overlap:
+ * the launch before it in the stream is a kernel, and (substep 2) the CFL words
+ * are clear already */
 cudaError_t launch_substep(Device d, cudaStream_t st, const int step, const double dt,
-                           unsigned long long* launches, const int zlo = 0, const int zhi = -1);
+                           unsigned long long* launches, const int zlo = 0, const int zhi = -1,
+                           const bool overlap = false);
 cudaError_t launch_periodic(Device d, cudaStream_t st, const int q0, const int nq,
-                            const Volume start, const Volume end, unsigned long long* launches);
+                            const Volume start, const Volume end, unsigned long long* launches,
+                            const bool overlap = false);
 void invalidate_tape_graph(Device d);

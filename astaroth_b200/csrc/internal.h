@@ -218,13 +218,52 @@ struct device_s {
     unsigned long long launches;
 };
 
+/* ---- overlapped launches within a step ----
+ * A kernel launched with `overlap` may start while the kernel before it in the
+ * stream still runs (programmatic dependent launch): it sets itself up, then
+ * ac_wait_predecessor() waits until that kernel is complete and its writes are
+ * visible.  Only for a launch whose predecessor in the stream is a kernel; a
+ * kernel must call ac_wait_predecessor() before its first access to memory that
+ * another kernel writes or reads. */
+#ifdef __CUDACC__
+__device__ __forceinline__ void
+ac_let_successor_start()
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+__device__ __forceinline__ void
+ac_wait_predecessor()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... K, typename... A>
+inline cudaError_t
+ac_launch_overlapped(void (*kernel)(K...), const dim3 grid, const dim3 block, const size_t smem,
+                     cudaStream_t stream, const bool overlap, A&&... args)
+{
+    cudaLaunchAttribute attr;
+    attr.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c                            = {};
+    c.gridDim                                       = grid;
+    c.blockDim                                      = block;
+    c.dynamicSmemBytes                              = smem;
+    c.stream                                        = stream;
+    c.attrs                                         = &attr;
+    c.numAttrs                                      = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, K(args)...);
+}
+#endif
+
 /* ---- launchers (each returns the launch error, cudaSuccess on success) ---- */
 
 /* Periodic halo fill of n arrays of element type T (double or float). */
 template <typename T>
 cudaError_t ac_launch_periodic(const Geom& g, T* const* arrays, const int n, const Volume start,
                                const Volume end, cudaStream_t stream,
-                               unsigned long long* launches);
+                               unsigned long long* launches,
+                               const bool overlap = false);
 
 cudaError_t ac_launch_fill(double* ptr, const long long count, const double value,
                            cudaStream_t stream, unsigned long long* launches);
@@ -301,12 +340,14 @@ cudaError_t ac_launch_solve_split64(const Geom& g, const SplitBufferMaps& in,
                                     const SplitBufferMaps& out, const Fields64& f,
                                     const StencilCoef& sc, const PhysConst& pc, const RkCoef& rk,
                                     int* err, unsigned long long* cfl, cudaStream_t stream,
-                                    unsigned long long* launches, const int sms = AC_SMS);
+                                    unsigned long long* launches, const int sms = AC_SMS,
+                                    const bool overlap = false);
 cudaError_t ac_launch_solve_split32(const Geom& g, const SplitBufferMaps& in,
                                     const SplitBufferMaps& out, const Fields32& f,
                                     const StencilCoef& sc, const PhysConst& pc, const RkCoef& rk,
                                     int* err, unsigned long long* cfl, cudaStream_t stream,
-                                    unsigned long long* launches, const int sms = AC_SMS);
+                                    unsigned long long* launches, const int sms = AC_SMS,
+                                    const bool overlap = false);
 /* the z chunk that the tap kernel takes for a whole mesh: 32 and more above about 96^3 */
 int ac_taps_zchunk(const Geom& g, const int precision);
 bool ac_tiled_supported(const Geom& g, const int precision);

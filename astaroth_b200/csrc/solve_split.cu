@@ -1043,6 +1043,9 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
     tmem::fence_before_sync();
     __syncthreads();
     tmem::fence_after_sync();
+    /* the set-up above overlaps the end of the halo fill (ac_launch_overlapped) */
+    ac_let_successor_start();
+    ac_wait_predecessor();
     const uint32_t tbase = *tslot;
     ch.tl                = tmem::lane_base(tbase, warp);
     ch.rfull             = bars;
@@ -1148,7 +1151,7 @@ cudaError_t
 launch_split(const Geom& g, const SplitMaps& tm, const FieldsT<T>& f, const StencilCoef& sc,
              const PhysConst& pc, const RkCoef& rk, int* err, unsigned long long* cfl,
              cudaStream_t stream, unsigned long long* launches, const int sms,
-             [[maybe_unused]] const bool threads_load)
+             [[maybe_unused]] const bool threads_load, const bool overlap)
 {
     typedef SplitTile<V> S;
     const int nzr = pc.zhi - pc.zlo;
@@ -1164,9 +1167,10 @@ launch_split(const Geom& g, const SplitMaps& tm, const FieldsT<T>& f, const Sten
     r.beta = Pack<V>::dup(rk.beta);
     r.ab   = Pack<V>::dup(rk.ab);
     const bool sum = pc.cfl_sum != 0, skip = pc.debug_skip_load != 0;
+    cudaError_t e = cudaSuccess;
     auto launch = [&](auto kernel) {
-        kernel<<<bpg, tpb, S::SMEM_BYTES, stream>>>(tm, g, f, c, r, pc.zlo, pc.zhi, zc, err, cfl, sum,
-                                                    (T)pc.cs2_sound, skip);
+        e = ac_launch_overlapped(kernel, bpg, tpb, S::SMEM_BYTES, stream, overlap, tm, g, f, c, r,
+                                 pc.zlo, pc.zhi, zc, err, cfl, sum, (T)pc.cs2_sound, skip);
     };
     auto pick = [&](auto ldg) {
         constexpr bool LDG = decltype(ldg)::value;
@@ -1187,7 +1191,7 @@ launch_split(const Geom& g, const SplitMaps& tm, const FieldsT<T>& f, const Sten
         pick(std::false_type{});
     if (launches)
         ++*launches;
-    return cudaGetLastError();
+    return e;
 }
 
 template <typename V>
@@ -1264,18 +1268,18 @@ cudaError_t
 ac_launch_solve_split64(const Geom& g, const SplitBufferMaps& in, const SplitBufferMaps& out, const Fields64& f,
                         const StencilCoef& sc, const PhysConst& pc, const RkCoef& rk, int* err,
                         unsigned long long* cfl, cudaStream_t stream, unsigned long long* launches,
-                        const int sms)
+                        const int sms, const bool overlap)
 {
     return launch_split<double>(g, SplitMaps{in.plane, out.tile, out.tile_lo, in.tile_lo}, f, sc, pc,
-                                rk, err, cfl, stream, launches, sms, in.threads_load);
+                                rk, err, cfl, stream, launches, sms, in.threads_load, overlap);
 }
 
 cudaError_t
 ac_launch_solve_split32(const Geom& g, const SplitBufferMaps& in, const SplitBufferMaps& out, const Fields32& f,
                         const StencilCoef& sc, const PhysConst& pc, const RkCoef& rk, int* err,
                         unsigned long long* cfl, cudaStream_t stream, unsigned long long* launches,
-                        const int sms)
+                        const int sms, const bool overlap)
 {
     return launch_split<F2>(g, SplitMaps{in.plane, out.tile, out.tile_lo, in.tile_lo}, f, sc, pc,
-                                rk, err, cfl, stream, launches, sms, in.threads_load);
+                                rk, err, cfl, stream, launches, sms, in.threads_load, overlap);
 }
