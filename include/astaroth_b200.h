@@ -97,11 +97,10 @@ typedef enum {
      * 1 = additive (min over cells of the local dt). */
     AC_additive_timestep,
     /* Selects the solve kernel (for tests and timing): 0 = the default (the
-     * leading-plane tiled kernel on z chunks of 32 planes and more, else the
-     * per-plane tap tiled kernel), 1 = the plain (untiled) kernel, 2 = the tiled
-     * kernel that reads every stencil tap of plane z from shared memory, 3 = the
-     * leading-plane tiled kernel, 4 = the same with the exchange between its
-     * warp groups through shared memory instead of tensor memory. */
+     * split-stage kernel where it takes the mesh, else the per-plane tap kernel,
+     * else the plain one), 1 = the plain (untiled) kernel, 2 = the tiled kernel
+     * that reads every stencil tap of plane z from shared memory, 3 and 4 = the
+     * split-stage kernel (as 0). */
     AC_debug_plain_kernel,
     /* Upwinding terms of the continuity and momentum equations when nonzero:
      * the reference's LUPWD build option (mhdsolver.ac:101,336-338,357-359;
