@@ -30,15 +30,11 @@ adj_geom(const Device d)
 static cudaError_t
 join_state(const Device d, cudaStream_t st, double* dst, unsigned long long* launches)
 {
-    const Geom g64 = adj_geom(d);
-    for (int q = 0; q < AC_NF; ++q) {
-        const int b          = d->in_idx[q];
-        const cudaError_t e  = ac_launch_join(d->geom, arr_hi(d, b, q), arr_lo(d, b, q),
-                                              dst + (size_t)q * g64.cells, st, launches);
-        if (e != cudaSuccess)
-            return e;
-    }
-    return cudaSuccess;
+    const size_t cells = (size_t)adj_geom(d).cells;
+    double* p[AC_NF];
+    for (int q = 0; q < AC_NF; ++q)
+        p[q] = dst + (size_t)q * cells;
+    return ac_launch_fields(d->geom, field_pairs(d, p), true, st, launches);
 }
 
 /* values of one slot array: the interior cells, an even number of them */
@@ -237,7 +233,7 @@ acDeviceAdjointTapeForward(const Device d, const Stream stream, const int steps,
         d->tape_stream[blk] = (int)stream;
     }
     AC_CUDA_CHECK(cudaGraphLaunch(d->tape_exec[blk], st));
-    d->launches += (d->precision == 0 ? 9ull : 33ull) * steps; /* FP32: 8 joins per state */
+    d->launches += 9ull * steps; /* halo fill, state to the tape, substep */
     d->out_set = 0;
     if ((3 * steps) & 1) /* three swaps per step */
         acDeviceSwapBuffers(d);

@@ -338,6 +338,19 @@ acDeviceCommitStagedMesh(const Device d, const Stream stream)
 
 /* ---- transfers from and to caller-owned device arrays ---- */
 
+/* Whether the eight fields lie one behind the other, as in a buffer block of an
+ * FP64 device, and the in-buffers are one block: one copy then moves them all. */
+static bool
+one_block(const Device d, const AcReal* const* p, const size_t n)
+{
+    if (d->precision != 0 || in_block_index(d) < 0)
+        return false;
+    for (int q = 1; q < AC_NF; ++q)
+        if (p[q] != p[0] + q * n)
+            return false;
+    return true;
+}
+
 extern "C" AcResult
 acDeviceLoadMeshDevice(const Device d, const Stream stream, const AcReal* const* src)
 {
@@ -345,17 +358,22 @@ acDeviceLoadMeshDevice(const Device d, const Stream stream, const AcReal* const*
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
     const size_t n = (size_t)d->geom.mx * d->geom.my * d->geom.mz;
-    for (int q = 0; q < AC_NF; ++q) {
+    for (int q = 0; q < AC_NF; ++q)
         if (!src[q])
             return AC_NOT_ALLOCATED;
-        const int b = d->in_idx[q];
-        if (d->precision == 0)
-            AC_CUDA_CHECK(cudaMemcpyAsync(arr64(d, b, q), src[q], n * sizeof(double),
-                                          cudaMemcpyDeviceToDevice, use_stream(d, stream)));
-        else
-            AC_CUDA_CHECK(ac_launch_split(d->geom, src[q], arr_hi(d, b, q), arr_lo(d, b, q),
-                                          use_stream(d, stream), &d->launches));
+    const cudaStream_t st = use_stream(d, stream);
+    if (d->precision != 0) {
+        double* p[AC_NF];
+        for (int q = 0; q < AC_NF; ++q)
+            p[q] = const_cast<double*>(src[q]); /* (read only) */
+        AC_CUDA_CHECK(ac_launch_fields(d->geom, field_pairs(d, p), false, st, &d->launches));
+        return AC_SUCCESS;
     }
+    const bool all = one_block(d, src, n);
+    for (int q = 0; q < (all ? 1 : AC_NF); ++q)
+        AC_CUDA_CHECK(cudaMemcpyAsync(arr64(d, d->in_idx[q], q), src[q],
+                                      (all ? AC_NF : 1) * n * sizeof(double),
+                                      cudaMemcpyDeviceToDevice, st));
     return AC_SUCCESS;
 }
 
@@ -366,17 +384,19 @@ acDeviceStoreMeshDevice(const Device d, const Stream stream, AcReal* const* dst)
         return AC_FAILURE;
     AC_CUDA_CHECK(cudaSetDevice(d->id));
     const size_t n = (size_t)d->geom.mx * d->geom.my * d->geom.mz;
-    for (int q = 0; q < AC_NF; ++q) {
+    for (int q = 0; q < AC_NF; ++q)
         if (!dst[q])
             return AC_NOT_ALLOCATED;
-        const int b = d->in_idx[q];
-        if (d->precision == 0)
-            AC_CUDA_CHECK(cudaMemcpyAsync(dst[q], arr64(d, b, q), n * sizeof(double),
-                                          cudaMemcpyDeviceToDevice, use_stream(d, stream)));
-        else
-            AC_CUDA_CHECK(ac_launch_join(d->geom, arr_hi(d, b, q), arr_lo(d, b, q), dst[q],
-                                         use_stream(d, stream), &d->launches));
+    const cudaStream_t st = use_stream(d, stream);
+    if (d->precision != 0) {
+        AC_CUDA_CHECK(ac_launch_fields(d->geom, field_pairs(d, dst), true, st, &d->launches));
+        return AC_SUCCESS;
     }
+    const bool all = one_block(d, dst, n);
+    for (int q = 0; q < (all ? 1 : AC_NF); ++q)
+        AC_CUDA_CHECK(cudaMemcpyAsync(dst[q], arr64(d, d->in_idx[q], q),
+                                      (all ? AC_NF : 1) * n * sizeof(double),
+                                      cudaMemcpyDeviceToDevice, st));
     return AC_SUCCESS;
 }
 

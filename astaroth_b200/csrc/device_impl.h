@@ -61,6 +61,19 @@ fields32(const Device d)
     return f;
 }
 
+/* the in-buffers of an FP32-compensated device with the doubles that d[] points at */
+static inline AcFieldPairs
+field_pairs(const Device dev, double* const* d)
+{
+    AcFieldPairs a;
+    for (int q = 0; q < AC_NF; ++q) {
+        a.d[q]  = d[q];
+        a.hi[q] = arr_hi(dev, dev->in_idx[q], q);
+        a.lo[q] = arr_lo(dev, dev->in_idx[q], q);
+    }
+    return a;
+}
+
 /* The block holding every field's in-buffer (0 or 1), or -1 when single
  * fields were swapped on their own. */
 static inline int

@@ -302,6 +302,14 @@ cudaError_t ac_launch_fill_comp(float* hi, float* lo, const long long count, con
 /* FP32 compensated <-> double (host layout, row pitch mx) conversions of one field */
 cudaError_t ac_launch_split(const Geom& g, const double* src, float* hi, float* lo,
                             cudaStream_t stream, unsigned long long* launches);
+/* all eight fields of a mesh in one launch: d (doubles) <-> (hi, lo) */
+struct AcFieldPairs {
+    double* d[AC_NF];
+    float* hi[AC_NF];
+    float* lo[AC_NF];
+};
+cudaError_t ac_launch_fields(const Geom& g, const AcFieldPairs& a, const bool join,
+                             cudaStream_t stream, unsigned long long* launches);
 cudaError_t ac_launch_join(const Geom& g, const float* hi, const float* lo, double* dst,
                            cudaStream_t stream, unsigned long long* launches);
 
