@@ -120,7 +120,7 @@ struct Pack<F2> {
     }
 };
 
-/* tensor-memory words of a value (tmem::Words) */
+/* tensor-memory words of a value */
 __device__ __forceinline__ void
 to_words(const double v, uint32_t* w)
 {

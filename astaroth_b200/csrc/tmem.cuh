@@ -79,7 +79,7 @@ lane_base(const uint32_t tbase, const int warp)
  * They touch tensor memory only, so they carry no memory clobber and ordinary
  * loads may be scheduled across them; being volatile, they keep their order
  * among themselves and with the waits.  A load's registers are valid only after
- * wait_ld_tied() on them. */
+ * wait_ld() and a tie of them to it (TWords::tie). */
 
 __device__ __forceinline__ void
 st1(const uint32_t a, const uint32_t v)
@@ -244,53 +244,5 @@ ld_n(const uint32_t a, uint32_t* v)
         ld1(a, v);
     }
 }
-
-/* Waits for this thread's loads, then ties the loaded words to the wait (an
- * empty volatile statement per word, after the wait in program order) so that
- * no use of them can be scheduled before it. */
-template <int N>
-__device__ __forceinline__ void
-wait_ld_tied(uint32_t* w)
-{
-    asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-        asm volatile("" : "+r"(w[i]));
-}
-
-/* A record of N values of type T as 32-bit words: N * sizeof(T) / 4 columns. */
-template <typename T, int N>
-struct Words {
-    static constexpr int W = N * (int)sizeof(T) / 4;
-    uint32_t w[W];
-    __device__ __forceinline__ void set(const int i, const T v)
-    {
-        if constexpr (sizeof(T) == 8) {
-            const unsigned long long b = (unsigned long long)__double_as_longlong((double)v);
-            w[2 * i]                   = (uint32_t)b;
-            w[2 * i + 1]               = (uint32_t)(b >> 32);
-        }
-        else {
-            w[i] = __float_as_uint((float)v);
-        }
-    }
-    __device__ __forceinline__ T get(const int i) const
-    {
-        if constexpr (sizeof(T) == 8)
-            return (T)__longlong_as_double((long long)(((unsigned long long)w[2 * i + 1] << 32) |
-                                                       (unsigned long long)w[2 * i]));
-        else
-            return (T)__uint_as_float(w[i]);
-    }
-    __device__ __forceinline__ void store(const uint32_t a) const { st_n<W>(a, w); }
-    __device__ __forceinline__ void load(const uint32_t a) { ld_n<W>(a, w); }
-    /* after this thread's wait::ld: ties the words to it */
-    __device__ __forceinline__ void tie()
-    {
-#pragma unroll
-        for (int i = 0; i < W; ++i)
-            asm volatile("" : "+r"(w[i]));
-    }
-};
 
 } // namespace tmem
