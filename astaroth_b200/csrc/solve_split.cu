@@ -393,14 +393,17 @@ struct Chunk {
 
 /* The end of an interval: this thread's tensor-memory accesses are ordered
  * before those that any thread makes after it, and the shared-memory slots read
- * in it are free.  (No memory clobber: tensor-memory accesses are volatile, and
- * shared memory is read behind an mbarrier wait.) */
+ * in it are free (the memory clobbers of the barrier and of the fences beside it
+ * keep the reads of a slot before its refill).  Called by a whole converged warp:
+ * the tensor-memory wait is warp-collective (.sync.aligned), as are the loads and
+ * stores, so a __syncwarp() stands between each of them and any code before it
+ * that single threads branch around. */
 __device__ __forceinline__ void
 interval_end()
 {
     tmem::wait_st();
     tmem::fence_before_sync();
-    asm volatile("bar.sync 0;");
+    asm volatile("bar.sync 0;" ::: "memory");
     tmem::fence_after_sync();
 }
 
@@ -585,6 +588,7 @@ inplane_role(const SplitMaps* maps, const SplitCoef<V>& c, const Chunk& ch,
         }
         rec = ++r5 == REC_SLOTS ? (r5 = 0, rec - (REC_SLOTS - 1) * TM::REC_W) : rec + TM::REC_W;
     }
+    __syncwarp();
     interval_end(); /* the last solve interval's exchange */
     return ok;
 }
@@ -783,6 +787,7 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
     uint32_t rec = ch.tl + r5 * TM::REC_W;
 #pragma unroll 1
     for (int i = 0; i < 7; ++i) {
+        __syncwarp(); /* after the copies, whose threads differ */
         interval_end();
         copy_plane(ch.pfirst + i + S::RING);
     }
@@ -795,6 +800,7 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
                 for (int k = 0; k < 4; ++k)
                     own[k] = f.out[k][i0];
             }
+        __syncwarp(); /* after the loads above and the last plane's stores: cells in the mesh only */
         TWords<4> w[7];
 #pragma unroll
         for (int k = 0; k < 7; ++k)
@@ -1088,6 +1094,7 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
         for (int p = ch.z0; p < ch.z0 + S::PRING; ++p)
             load_prev<V>(&maps, ch, smem, p, PREV, x0, y0);
     }
+    __syncwarp(); /* setmaxnreg is warp-collective */
 
     const int cell_off = (ly + NGHOST) * S::HXP + (lx + NGHOST);
     const int x = x0 + lx, y = y0 + ly;

@@ -74,3 +74,15 @@ def test_z_boxes_of_any_size_give_the_same_bits():
             out.append((d.store_mesh(), d.timestep_maxima()))
     for o, m in out[1:]:
         assert np.array_equal(o, out[0][0]) and m == out[0][1]
+
+
+@pytest.mark.parametrize("precision,n", [(0, (37, 7, 40)), (0, (38, 7, 40)), (1, (38, 11, 40))])
+def test_ragged_tiles_give_the_same_bits_every_time(precision, n):
+    """Tiles that reach past the mesh in x and y, where the threads of a warp part at
+    the loads, copies and stores of cells that the mesh does not have and have to be
+    together again at the tensor-memory accesses that follow: planes by TMA and (odd
+    nx) by the threads, with and without a previous state."""
+    first, _, _ = run(n, precision, 0)
+    for _ in range(10):
+        again, _, _ = run(n, precision, 0)
+        assert np.array_equal(again, first)
