@@ -338,8 +338,31 @@ acDeviceCommitStagedMesh(const Device d, const Stream stream)
 
 /* ---- transfers from and to caller-owned device arrays ---- */
 
-/* Whether the eight fields lie one behind the other, as in a buffer block of an
- * FP64 device, and the in-buffers are one block: one copy then moves them all. */
+/* Whether [p, p + bytes) lies in one allocation, as the driver knows it (false
+ * where it does not say). */
+static bool
+one_allocation(const void* p, const size_t bytes)
+{
+    typedef CUresult (*RangeFn)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const RangeFn range = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool found = cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault,
+                                                   &q) == cudaSuccess &&
+                           q == cudaDriverEntryPointSuccess;
+        return found ? (RangeFn)fn : nullptr;
+    }();
+    CUdeviceptr base = 0;
+    size_t size      = 0;
+    return range && range(&base, &size, (CUdeviceptr)p) == CUDA_SUCCESS &&
+           (CUdeviceptr)p - base <= size && bytes <= size - ((CUdeviceptr)p - base);
+}
+
+/* Whether the eight fields lie one behind the other in one allocation, as in a
+ * buffer block of an FP64 device, and the in-buffers are one block: one copy then
+ * moves them all.  (The addresses alone do not say it: arrays allocated one by
+ * one can be neighbours, at 58^3 cells of exactly 2 MiB for instance, and a copy
+ * may not run from one allocation into the next.) */
 static bool
 one_block(const Device d, const AcReal* const* p, const size_t n)
 {
@@ -348,7 +371,7 @@ one_block(const Device d, const AcReal* const* p, const size_t n)
     for (int q = 1; q < AC_NF; ++q)
         if (p[q] != p[0] + q * n)
             return false;
-    return true;
+    return one_allocation(p[0], AC_NF * n * sizeof(AcReal));
 }
 
 extern "C" AcResult

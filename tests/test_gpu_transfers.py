@@ -208,3 +208,53 @@ def test_staged_loads_overlap_and_equal_direct_loads(precision):
         d.transfer_mesh(e)
         d.synchronize()
         assert np.array_equal(e.store_mesh(), direct[1])
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_device_arrays_allocated_one_by_one(precision):
+    """Eight arrays of exactly 2 MiB (58^3 cells with their halo), each an allocation
+    of its own, where possible neighbours in address order: the mesh goes in and out,
+    and what lies around the arrays stays as it was."""
+    import torch  # loads the CUDA runtime
+
+    torch.cuda.synchronize()
+    rt = C.CDLL("libcudart.so.12")
+    rt.cudaMemcpy.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
+    rt.cudaFree.argtypes = [C.c_void_p]
+    info = ab.make_info(58, precision=precision, **ab.CONFIG_PARAMS)
+    f = ab.seeded_mesh(info, 12)
+    nbytes = f[0].nbytes
+    assert nbytes == 2 << 20
+    ptrs = []
+    for _ in range(32):
+        p = C.c_void_p()
+        assert rt.cudaMalloc(C.byref(p), C.c_size_t(nbytes)) == 0
+        ptrs.append(p.value)
+    try:
+        ptrs.sort()
+        run = next((i for i in range(len(ptrs) - 7) if ptrs[i + 7] - ptrs[i] == 7 * nbytes), 0)
+        eight, rest = ptrs[run:run + 8], ptrs[:run] + ptrs[run + 8:]
+        mark = np.full_like(f[0], 7.25)
+        for p in rest:
+            assert rt.cudaMemcpy(p, mark.ctypes.data, nbytes, 1) == 0
+        for q, p in enumerate(eight):
+            assert rt.cudaMemcpy(p, f[q].ctypes.data, nbytes, 1) == 0
+        arrays = (C.c_void_p * 8)(*eight)
+        lib = capi.load()
+        with ab.Device(info) as d:
+            assert lib.acDeviceLoadMeshDevice(d.handle, 0, arrays) == 0
+            d.synchronize()
+            assert np.array_equal(d.store_mesh(), _held(f, precision))
+            d.load_mesh(-f)
+            assert lib.acDeviceStoreMeshDevice(d.handle, 0, arrays) == 0
+            d.synchronize()
+        back = np.empty_like(f[0])
+        for q, p in enumerate(eight):
+            assert rt.cudaMemcpy(back.ctypes.data, p, nbytes, 2) == 0
+            assert np.array_equal(back, -_held(f[q], precision))
+        for p in rest:
+            assert rt.cudaMemcpy(back.ctypes.data, p, nbytes, 2) == 0
+            assert np.array_equal(back, mark)
+    finally:
+        for p in ptrs:
+            rt.cudaFree(p)
