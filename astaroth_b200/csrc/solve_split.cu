@@ -123,10 +123,11 @@ struct SplitMaps {
 template <typename V>
 struct SplitCoef {
     V d1[3][3];  /* first derivative, [axis][k-1] */
-    V d2[3][3];  /* second derivative sides, [axis][k-1] */
-    V d2c[3];    /* its centre */
-    V c_all;     /* d2c[0] + d2c[1] + d2c[2] */
-    V c_xy, c_yz, c_xz;
+    /* Laplacians of lnrho and s, and of A, each in a unit of its own (lap_unit; FP64: 1)
+     * that the factors gicp_l, gm1_l and eta, nim take back: sides, [axis][k-1]; centres of
+     * all axes; A: centres of two axes, and what av_c[a] adds to that of the other two */
+    V sd2[3][3], s_all;
+    V ad2[3][3], a_xy, a_yz, a_xz, av_c[3];
     /* hydro: nu lap u_c + vg d/dx_c div u, vg = nu/3 + zeta */
     V vd[3][3]; /* (nu + vg) d2 sides: axis c of component c */
     V vn[3][3]; /* nu d2 sides: the other axes */
@@ -139,24 +140,67 @@ struct SplitCoef {
     /* magnetic: j = (grad div A - lap A) / mu0 */
     V mm[3][3]; /* mix / mu0 */
     V mmn[2][3];
-    V nim;      /* -1/mu0 */
+    V nim;      /* -1/mu0, in the unit of lap A */
     V up[3][4]; /* upwinding, [axis][k]: centre and sides */
     /* equations */
-    V m23, two, one_half, two_nu, nu, inv_cp, ncs2, gicp, gm1, gm1_lnrho0, inv_exp_lnT0, eta, eta_mu0,
-        zeta, K;
+    V m23, two, one_half, nu, inv_cp, ncs2, gicp, gm1, gicp_l, gm1_l, gm1_lnrho0, inv_exp_lnT0, eta,
+        eta_mu0, zeta, K;
 };
+
+/* v over what FP32 holds of it */
+inline double
+made_up(const double v)
+{
+    const double r = v / (double)(float)v;
+    return r > 0.5 && r < 2 ? r : 1; /* (1 for zero and for what FP32 does not hold) */
+}
+
+/* FP32: a unit for Laplacians that are only used times fa and fb.  The sides of an
+ * isotropic mesh are 270, -27 and 2 in units of 1/(180 dx^2) and the centre is -1470, so
+ * that in 1/m of it, m a whole number, all of them are FP32 numbers and a constant has no
+ * Laplacian: only fa and fb times the unit are rounded, and m is the one of 32 for which
+ * these are rounded least (to about 5e-9 of themselves).  Rounded at 1/ds^2 every
+ * coefficient was off by up to 6e-8, by chance of the spacing, and a constant had a
+ * Laplacian of 5e-7 / ds^2 of its value at 512^3 (entropy 3.0e-7 off FP64 after 100 steps). */
+inline long double
+lap_unit(const StencilCoef& s, const double fa, const double fb)
+{
+    const double base = s.d2[0][1] / 270;
+    double least      = 1;
+    int best          = 1;
+    for (int m = 1; m <= 32; ++m) {
+        const double off = fmax(fabs(made_up(fa * base / m) - 1), fabs(made_up(fb * base / m) - 1));
+        if (off < least) {
+            least = off;
+            best  = m;
+        }
+    }
+    return (long double)base / best;
+}
 
 template <typename V>
 SplitCoef<V>
-make_coef(const StencilCoef& s, const PhysConst& p)
+make_coef(const StencilCoef& s, const PhysConst& p, const RkCoef& rk)
 {
     SplitCoef<V> c;
     auto D          = [](const long double v) { return Pack<V>::dup((double)v); };
-    const long double nu = p.nu, vg = (long double)p.nu / 3 + p.zeta, im = p.inv_mu0;
+    constexpr bool FP32 = Pack<V>::N == 2;
+    /* FP32: an increment is beta dt times a rate, beta and dt each rounded.  The factors of
+     * the rates that are rounded anyhow make up for that, and ab for beta's part (lnrho,
+     * whose rate has no factors, keeps the rounding of dt).  With it u, A and s end a run half
+     * as far off FP64, over the sizes and options of 44 runs (100 steps at 512^3: u 1.0e-7,
+     * A 5.9e-8, s 7.9e-8; each factor rounded by itself 1.4e-7, 3.5e-7, 3.0e-7) */
+    const double t = FP32 ? made_up(rk.beta) * made_up(rk.dt) : 1;
+    const long double nu = p.nu * t, vg = ((long double)p.nu / 3 + p.zeta) * t, im = p.inv_mu0;
+    /* K multiplies the Laplacians of lnrho and s too: their factors make up for its rounding */
+    const double kr      = FP32 ? made_up(p.K * t) : 1;
+    const long double us = FP32 ? lap_unit(s, p.gamma_inv_cp * kr, p.gamma_m1 * kr) : 1;
+    const long double ua = FP32 ? lap_unit(s, p.eta * t, p.inv_mu0) : 1;
     for (int a = 0; a < 3; ++a) {
         for (int k = 0; k < 3; ++k) {
             c.d1[a][k] = D(s.d1[a][k]);
-            c.d2[a][k] = D(s.d2[a][k + 1]);
+            c.sd2[a][k] = D(s.d2[a][k + 1] / us);
+            c.ad2[a][k] = D(s.d2[a][k + 1] / ua);
             c.vd[a][k] = D((nu + vg) * s.d2[a][k + 1]);
             c.vn[a][k] = D(nu * s.d2[a][k + 1]);
             c.vm[a][k] = D(vg * s.mix[a][k]);
@@ -166,12 +210,11 @@ make_coef(const StencilCoef& s, const PhysConst& p)
                 c.mmn[a - 1][k] = D(-im * s.mix[a][k]);
             }
         }
-        c.d2c[a] = D(s.d2[a][0]);
         for (int k = 0; k < 4; ++k)
             c.up[a][k] = D(s.up[a][k]);
         c.vc[a]  = D(nu * ((long double)s.d2[0][0] + s.d2[1][0] + s.d2[2][0]) + vg * s.d2[a][0]);
     }
-    if (Pack<V>::N == 2)
+    if (FP32)
         for (int q = 0; q < 3; ++q) {
             long double sides = 0; /* of the FP32 coefficients */
             for (int a = 0; a < 3; ++a)
@@ -182,26 +225,43 @@ make_coef(const StencilCoef& s, const PhysConst& p)
                                            vg * s.d2[q][0]);
             c.vcl[q] = D(-sides - (long double)(float)centre);
         }
-    c.c_all = D((long double)s.d2[0][0] + s.d2[1][0] + s.d2[2][0]);
-    c.c_xy  = D((long double)s.d2[0][0] + s.d2[1][0]);
-    c.c_yz  = D((long double)s.d2[1][0] + s.d2[2][0]);
-    c.c_xz  = D((long double)s.d2[0][0] + s.d2[2][0]);
-    c.nim          = D(-im);
+    /* centres: FP64 the sums of the three axes'; FP32 minus the sums of the rounded sides,
+     * rounded once (they differ where the spacings do) */
+    auto in_T    = [](const long double v) { return (long double)(typename Pack<V>::T)(double)v; };
+    auto centre  = [&](const int a, const long double u) {
+        long double v = s.d2[a][0];
+        if (FP32) {
+            v = 0;
+            for (int k = 1; k <= 3; ++k)
+                v -= 2 * in_T(s.d2[a][k] / u);
+        }
+        return v;
+    };
+    const long double ax = centre(0, ua), ay = centre(1, ua), az = centre(2, ua);
+    c.s_all = D(centre(0, us) + centre(1, us) + centre(2, us));
+    c.a_xy  = D(ax + ay);
+    c.a_yz  = D(ay + az);
+    c.a_xz  = D(ax + az);
+    c.av_c[0] = D(FP32 ? ax + ay + az - in_T(ay + az) : ax);
+    c.av_c[1] = D(FP32 ? ax + ay + az - in_T(ax + az) : ay);
+    c.av_c[2] = D(FP32 ? ax + ay + az - in_T(ax + ay) : az);
+    c.nim          = D(-im * ua);
     c.m23          = D(-2.0L / 3);
     c.two          = D(2);
     c.one_half     = D(0.5);
-    c.two_nu       = D(2 * nu);
     c.nu           = D(nu);
     c.inv_cp       = D(p.inv_cp);
-    c.ncs2         = D(-p.cs2_sound);
+    c.ncs2         = D(-p.cs2_sound * t);
     c.gicp         = D(p.gamma_inv_cp);
     c.gm1          = D(p.gamma_m1);
+    c.gicp_l       = D(p.gamma_inv_cp * kr * us);
+    c.gm1_l        = D(p.gamma_m1 * kr * us);
     c.gm1_lnrho0   = D(-(long double)p.gamma_m1 * p.lnrho0);
     c.inv_exp_lnT0 = D(p.inv_exp_lnT0);
-    c.eta          = D(p.eta);
-    c.eta_mu0      = D(p.eta_mu0);
-    c.zeta         = D(p.zeta);
-    c.K            = D(p.K);
+    c.eta          = D(p.eta * t * ua);
+    c.eta_mu0      = D(p.eta_mu0 * t);
+    c.zeta         = D(p.zeta * t);
+    c.K            = D(p.K * t);
     return c;
 }
 
@@ -491,7 +551,7 @@ inplane_role(const SplitMaps* maps, const SplitCoef<V>& c, const Chunk& ch,
                 upwind(0, vs);
                 r.set(H_SX, dot3(dx, c.d1[0]));
                 r.set(H_SY, dot3(dy, c.d1[1]));
-                r.set(H_SL, dot3p(sy, c.d2[1], dot3p(sx, c.d2[0], c.c_all * vs)));
+                r.set(H_SL, dot3p(sy, c.sd2[1], dot3p(sx, c.sd2[0], c.s_all * vs)));
                 taps_xy(t0, dx, sx, dy, sy);
                 upwind(1, v0);
                 const V done = mixed_first(acc[2], dx, e1, n1);
@@ -520,27 +580,27 @@ inplane_role(const SplitMaps* maps, const SplitCoef<V>& c, const Chunk& ch,
                 taps_xy(ts, dx, sx, dy, sy);
                 set(M_SX, dot3(dx, c.d1[0]));
                 set(M_SY, dot3(dy, c.d1[1]));
-                set(M_SL, dot3p(sy, c.d2[1], dot3p(sx, c.d2[0], c.c_all * vs)));
+                set(M_SL, dot3p(sy, c.sd2[1], dot3p(sx, c.sd2[0], c.s_all * vs)));
                 taps_xy(t0, dx, sx, dy, sy);
                 const V done = mixed_first(acc[2], dx, e1, n1);
                 const V dyAx = dot3(dy, c.d1[1]);
                 {
-                    const V Y = dot3p(sy, c.d2[1], c.c_yz * v0);
-                    set(M_L0, dot3p(sx, c.d2[0], vfma(c.d2c[0], v0, Y)));
+                    const V Y = dot3p(sy, c.ad2[1], c.a_yz * v0);
+                    set(M_L0, dot3p(sx, c.ad2[0], vfma(c.av_c[0], v0, Y)));
                     set(M_Q0, dxy(t1, c.mm[0], c.nim * Y));
                 }
                 taps_xy(t1, dx, sx, dy, sy);
                 fin.set(2, mixed_second(acc[2], done, dy, e2, n2));
                 {
-                    const V X = dot3p(sx, c.d2[0], c.c_xz * v1);
-                    set(M_L1, dot3p(sy, c.d2[1], vfma(c.d2c[1], v1, X)));
+                    const V X = dot3p(sx, c.ad2[0], c.a_xz * v1);
+                    set(M_L1, dot3p(sy, c.ad2[1], vfma(c.av_c[1], v1, X)));
                     set(M_Q1, dxy(t0, c.mm[0], c.nim * X));
                 }
                 set(M_BZ, dot3(dx, c.d1[0]) - dyAx);
                 taps_xy(t2, dx, sx, dy, sy);
                 fin.set(0, mixed_first(acc[0], dx, e1, n1));
                 fin.set(1, mixed_first(acc[1], dy, e2, n2));
-                set(M_L2, dot3p(sy, c.d2[1], dot3p(sx, c.d2[0], c.c_xy * v2)));
+                set(M_L2, dot3p(sy, c.ad2[1], dot3p(sx, c.ad2[0], c.a_xy * v2)));
                 set(M_DXAZ, dot3(dx, c.d1[0]));
                 set(M_DYAZ, dot3(dy, c.d1[1]));
                 __syncwarp();
@@ -820,7 +880,7 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
             const V lnrho = w[3].template get<V>(0), ux = w[3].template get<V>(1), uy = w[3].template get<V>(2),
                     uz = w[3].template get<V>(3);
             V gl[3], gz[3], s2[4];
-            z_derivs(w, 0, c.d1[2], c.d2[2], gl[2], s2[0]);
+            z_derivs(w, 0, c.d1[2], c.sd2[2], gl[2], s2[0]);
             z_derivs(w, 1, c.d1[2], c.vn[2], gz[0], s2[1]);
             z_derivs(w, 2, c.d1[2], c.vn[2], gz[1], s2[2]);
             z_derivs(w, 3, c.d1[2], c.vd[2], gz[2], s2[3]);
@@ -925,10 +985,10 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
             uw.load(ch.tl + TM::ZQ0 + (uint32_t)(p & 7) * ZQ_W);
             const V ent = w[3].template get<V>(0);
             V gs[3], s2[4], dzAx, dzAy, unused;
-            z_derivs(w, 0, c.d1[2], c.d2[2], gs[2], s2[0]);
-            z_derivs(w, 1, c.d1[2], c.d2[2], dzAx, s2[1]);
-            z_derivs(w, 2, c.d1[2], c.d2[2], dzAy, s2[2]);
-            z_derivs(w, 3, c.d1[2], c.d2[2], unused, s2[3]);
+            z_derivs(w, 0, c.d1[2], c.sd2[2], gs[2], s2[0]);
+            z_derivs(w, 1, c.d1[2], c.ad2[2], dzAx, s2[1]);
+            z_derivs(w, 2, c.d1[2], c.ad2[2], dzAy, s2[2]);
+            z_derivs(w, 3, c.d1[2], c.ad2[2], unused, s2[3]);
             val[0] = w[3].template get<V>(1);
             val[1] = w[3].template get<V>(2);
             val[2] = w[3].template get<V>(3);
@@ -948,7 +1008,7 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
             const V j1 = vfma(c.nim, s2[2], R(M_Q1) + a.template get<V>(1));
             const V j2 = vfma(c.nim, l2, a.template get<V>(2));
             const V lap0 = R(M_L0) + s2[1], lap1 = R(M_L1) + s2[2];
-            const V lap2 = l2 + vfma(c.d2c[2], val[2], s2[3]);
+            const V lap2 = l2 + vfma(c.av_c[2], val[2], s2[3]);
             {
                 TWords<MX_N> xw;
                 xw.set(0, gs[0]);
@@ -989,7 +1049,7 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
             const V divu = hx.template get<V>(5);
             const V H    = vfma(irho * c.eta_mu0, jj,
                                 vfma(c.nu, hx.template get<V>(4), c.zeta * divu * divu));
-            V heat = vfma(c.gicp, laps, c.gm1 * hx.template get<V>(3));
+            V heat = vfma(c.gicp_l, laps, c.gm1_l * hx.template get<V>(3));
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
                 const V s = vfma(c.gicp, gs[q], c.gm1 * hx.template get<V>(q));
@@ -1192,11 +1252,11 @@ launch_split(const Geom& g, const SplitMaps& tm, const FieldsT<T>& f, const Sten
     const int zc = split_zchunk(bx * by, nzr, sms);
     const dim3 bpg(bx, by, (nzr + zc - 1) / zc);
     const dim3 tpb(TX, ROLES * WARPS_Y, 1);
-    const SplitCoef<V> c = make_coef<V>(sc, pc);
+    const SplitCoef<V> c = make_coef<V>(sc, pc, rk);
     RkV<V> r;
     r.dt   = Pack<V>::dup(rk.dt);
     r.beta = Pack<V>::dup(rk.beta);
-    r.ab   = Pack<V>::dup(rk.ab);
+    r.ab   = Pack<V>::dup(Pack<V>::N == 2 ? rk.ab * made_up(rk.beta) : rk.ab);
     const bool sum = pc.cfl_sum != 0, skip = pc.debug_skip_load != 0;
     cudaError_t e = cudaSuccess;
     auto launch = [&](auto kernel) {

@@ -86,3 +86,31 @@ def test_ragged_tiles_give_the_same_bits_every_time(precision, n):
     for _ in range(10):
         again, _, _ = run(n, precision, 0)
         assert np.array_equal(again, first)
+
+
+def test_fp32_laplacian_of_a_constant():
+    """The FP32 coefficients of the Laplacians cancel on a constant as well as FP32 allows.
+
+    A slow large-scale entropy profile about 1 under strong conduction, FP32-compensated
+    against FP64: a rounding of a cell's Laplacian has either sign, so that over the mesh
+    only what the coefficients leave of s itself is seen.  FP32 leaves at most half an ulp
+    of the centre, 3 * 49/18 / ds^2 = 848 at 64^3 (half an ulp: 3.05e-5), times s <= 1.25;
+    a rate is K exp(-lnrho) gamma/cp of it, with exp(-lnrho) <= 1.01 here.  Beside that,
+    the mean of 64^3 roundings in 30 substeps: 8 roundings of up to 6e-8 * 848 each,
+    / sqrt(64^3), is below 1e-6."""
+    n, steps, dt, K = 64, 10, 5e-4, 0.05
+    out = []
+    for precision in (0, 1):
+        info = make_info(n, precision=precision, **dict(CONFIG_PARAMS, K_heatcond=K))
+        f = np.zeros_like(seeded_mesh(info, 1))
+        x = (np.arange(n + 6) - 3) * (2 * np.pi / n)
+        f[7] = 1.0 + 0.25 * np.sin(x)[None, None, :] * np.cos(x)[None, :, None] * np.cos(x)[:, None, None]
+        with Device(info) as d:
+            d.load_mesh(f)
+            for _ in range(steps):
+                d.integrate_step(dt)
+            d.synchronize()
+            out.append(d.store_mesh()[:, 3:-3, 3:-3, 3:-3].copy())
+    drift = float((out[1][7] - out[0][7]).mean())
+    rate = K * 1.01 * CONFIG_PARAMS["gamma"] / CONFIG_PARAMS["cp_sound"]
+    assert abs(drift) <= steps * dt * rate * (3.05e-5 * 1.25 + 1e-6), drift
