@@ -783,8 +783,10 @@ launch_substep(Device d, cudaStream_t st, const int step, const double dt,
         }
         cfl = d->cfl;
     }
-    const bool split = d->solve_variant != 0 && d->split_ok && blk >= 0 &&
-                       d->solve_variant != AC_SOLVE_TILED_TAPS;
+    const bool split = d->split_ok && blk >= 0 &&
+                       (d->solve_variant == AC_SOLVE_TILED_SPLIT ||
+                        (d->solve_variant == AC_SOLVE_TILED_AUTO &&
+                         d->smaps[blk].automatic[pc.upwind != 0]));
     cudaError_t e;
     if (d->precision == 0) {
         const Fields64 f = fields64(d);

@@ -719,7 +719,8 @@ acEnsembleCreate(const int device_id, const int n, const AcMeshInfo* member_info
                                            : const_cast<float*>(members<float>(e)[m].f[p].in_lo[0]);
             if (!ac_make_tensor_map(&e->tmaps[2 * m + p], base, e->geom[m], e->precision))
                 e->tiled[m] = 0;
-            if (!ac_make_split_maps(&e->smaps[2 * m + p], base, lo, e->geom[m], e->precision))
+            if (!ac_make_split_maps(&e->smaps[2 * m + p], base, lo, e->geom[m], e->precision) ||
+                !e->smaps[2 * m + p].automatic[0]) /* (no upwinding here) */
                 e->split[m] = 0;
         }
     ENS_CHECK(ac_solve_tiled_init(e->precision));

@@ -156,6 +156,8 @@ struct StepGraph {
 struct SplitBufferMaps {
     CUtensorMap plane, tile, tile_lo;
     int threads_load; /* no maps: the kernel's threads load the planes */
+    int automatic[2]; /* the automatic choice takes the kernel for this mesh (without and
+                       * with upwinding) */
 };
 
 /* The two buffers of every field: block b holds all 8 fields of buffer b
@@ -332,8 +334,9 @@ cudaError_t ac_launch_reduce(const Geom& g, const void* const* fields, const flo
 int ac_reduce_blocks(const Geom& g);
 
 /* Tiled substep kernels: the split-stage kernel (solve_split.cu), which the
- * automatic choice takes for every mesh it fits, and the per-plane tap kernel
- * (solve_tiled.cu) for the others. */
+ * automatic choice takes for the meshes it fits (SplitBufferMaps::automatic: but
+ * for small FP64 ones with nx odd), and the per-plane tap kernel (solve_tiled.cu)
+ * for the others. */
 enum {
     AC_SOLVE_TILED_AUTO  = 1,
     AC_SOLVE_TILED_TAPS  = 2,

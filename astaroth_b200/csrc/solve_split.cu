@@ -1221,7 +1221,7 @@ solve_split_kernel(const __grid_constant__ SplitMaps maps, const Geom g,
  * solve roles' lag); the longest chunks on a tie.  Small meshes so come out as
  * one wave of short chunks, large ones as few long ones. */
 int
-split_zchunk(const int tiles, const int nz, const int sms)
+split_zchunk(const int tiles, const int nz, const int sms, long long* intervals = nullptr)
 {
     int best       = nz;
     long long cost = 0;
@@ -1234,7 +1234,26 @@ split_zchunk(const int tiles, const int nz, const int sms)
             best = zc;
         }
     }
+    if (intervals)
+        *intervals = cost;
     return best;
+}
+
+/* Whether the automatic choice takes this kernel with planes loaded by the threads (FP64,
+ * nx odd) and not the plain kernel.  Both have the same tiles.  A block here takes about
+ * 1.25 us an interval; the plain kernel, one plane a block and two blocks per SM, about
+ * 4.3 us (6.2 with upwinding) for as many as fit the GPU: at its best where the mesh is
+ * small or a few planes thin.  Per substep, plain / this: 33^3 12.5 / 15.6 us,
+ * 125 x 13 x 9 6.3 / 10.5, 255 x 255 x 3 26 / 43, 65^3 47 / 52; 73^3 58 / 58,
+ * 35 x 40 x 100 31 / 29, 103^3 183 / 123; this over plain with upwinding: 33^3 1.16,
+ * 39^3 0.96, 49^3 0.85. */
+bool
+split_beats_plain(const Geom& g, const bool upwind)
+{
+    const int tiles = (g.nx + TX - 1) / TX * ((g.ny + WARPS_Y - 1) / WARPS_Y);
+    long long intervals;
+    split_zchunk(tiles, g.nz, AC_SMS, &intervals);
+    return intervals <= (upwind ? 5.0 : 3.5) * tiles * g.nz / (2.0 * AC_SMS);
 }
 
 template <typename V, typename T>
@@ -1323,8 +1342,10 @@ ac_make_split_maps(SplitBufferMaps* m, void* hi, float* lo, const Geom& g, const
     typedef SplitTile<F2> F;
     /* FP64 rows of an odd number of values are no multiple of 16 bytes: no tensor
      * map, the threads load the planes.  125^3: 0.56 ms per step, the plain kernel
-     * 0.90 (128^3 by TMA 0.46). */
+     * 0.90 (128^3 by TMA 0.46); which of the two is faster depends on the size. */
     m->threads_load = precision == 0 && (g.nx & 1) && g.nx >= TX && g.ny >= WARPS_Y;
+    for (int upwind = 0; upwind < 2; ++upwind)
+        m->automatic[upwind] = !m->threads_load || split_beats_plain(g, upwind != 0);
     if (m->threads_load)
         return true;
     if (!ac_tiled_supported(g, precision) || g.my < (precision == 0 ? D::HY : F::HY))

@@ -1,4 +1,4 @@
-"""The split-stage substep kernel (the automatic choice) against the plain kernel
+"""The split-stage substep kernel against the plain kernel
 at the sizes where its tiles, chunks and queues have their edges: one tile and
 one cell more or less, chunks of a few planes, rows of the packed FP32 tile that
 lie outside the mesh.  Both evaluate the same equations with their sums in
@@ -37,7 +37,7 @@ def run(n, precision, kernel, **params):
 @pytest.mark.parametrize("n", SIZES)
 def test_split_kernel_equals_plain(n, precision):
     a, ma, _ = run(n, precision, 1)
-    b, mb, _ = run(n, precision, 0)
+    b, mb, _ = run(n, precision, 3)
     scale = np.abs(a).reshape(8, -1).max(axis=1)
     err = np.abs(a - b).reshape(8, -1).max(axis=1) / scale
     assert err.max() <= (1e-14 if precision == 0 else 6e-6), err
@@ -48,16 +48,17 @@ def test_split_kernel_equals_plain(n, precision):
 @pytest.mark.parametrize("n", [(65, 6, 5), (34, 7, 5), (66, 16, 11), (150, 13, 17)])
 def test_split_kernel_equals_plain_with_upwinding(n, precision):
     a, ma, _ = run(n, precision, 1, upwind=1)
-    b, mb, _ = run(n, precision, 0, upwind=1)
+    b, mb, _ = run(n, precision, 3, upwind=1)
     err = np.abs(a - b).reshape(8, -1).max(axis=1) / np.abs(a).reshape(8, -1).max(axis=1)
     assert err.max() <= (1e-14 if precision == 0 else 6e-6), err
     np.testing.assert_allclose(ma, mb, rtol=1e-13 if precision == 0 else 6e-6)
 
 
-def test_z_boxes_of_any_size_give_the_same_bits():
+@pytest.mark.parametrize("n", [(40, 12, 19), (41, 12, 19)])
+def test_z_boxes_of_any_size_give_the_same_bits(n):
     """Chunks start and end anywhere: the planes of a substep solved in uneven z boxes."""
-    n = (40, 12, 19)
     info = make_info(n, **CONFIG_PARAMS)
+    info.int_params[capi.IntParam.AC_debug_plain_kernel] = 3
     f = seeded_mesh(info, 5, **AMP)
     out = []
     for cuts in ((0, 19), (0, 1, 3, 4, 11, 19), (0, 6, 13, 19)):
@@ -82,9 +83,9 @@ def test_ragged_tiles_give_the_same_bits_every_time(precision, n):
     the loads, copies and stores of cells that the mesh does not have and have to be
     together again at the tensor-memory accesses that follow: planes by TMA and (odd
     nx) by the threads, with and without a previous state."""
-    first, _, _ = run(n, precision, 0)
+    first, _, _ = run(n, precision, 3)
     for _ in range(10):
-        again, _, _ = run(n, precision, 0)
+        again, _, _ = run(n, precision, 3)
         assert np.array_equal(again, first)
 
 
@@ -114,3 +115,27 @@ def test_fp32_laplacian_of_a_constant():
     drift = float((out[1][7] - out[0][7]).mean())
     rate = K * 1.01 * CONFIG_PARAMS["gamma"] / CONFIG_PARAMS["cp_sound"]
     assert abs(drift) <= steps * dt * rate * (3.05e-5 * 1.25 + 1e-6), drift
+
+
+@pytest.mark.parametrize("n,upwind,split", [((33, 33, 33), 0, False), ((255, 12, 3), 0, False),
+                                            ((49, 49, 49), 0, False), ((49, 49, 49), 1, True),
+                                            ((35, 40, 100), 0, True), ((101, 64, 51), 0, True)])
+def test_automatic_choice_for_odd_nx(n, upwind, split):
+    """FP64 meshes with nx odd take the faster of the plain kernel (small meshes) and the
+    split-stage kernel, in whole steps, calls of the loop and z boxes alike."""
+    auto, _, _ = run(n, 0, 0, upwind=upwind)
+    assert np.array_equal(auto, run(n, 0, 3 if split else 1, upwind=upwind)[0])
+    assert not np.array_equal(auto, run(n, 0, 1 if split else 3, upwind=upwind)[0])
+    info = make_info(n, **dict(CONFIG_PARAMS, upwind=upwind))
+    with Device(info) as d:
+        d.load_mesh(seeded_mesh(info, 17, **AMP))
+        for _ in range(2):
+            for s in range(3):
+                d.periodic_boundconds()
+                for z0, z1 in ((0, 2), (2, n[2])):
+                    assert d.lib.acDeviceIntegrateSubstep(
+                        d.handle, 0, s, capi.Volume(3, 3, 3 + z0),
+                        capi.Volume(3 + n[0], 3 + n[1], 3 + z1), 1e-3) == 0
+                d.swap_buffers()
+        d.synchronize()
+        assert np.array_equal(auto, d.store_mesh()[:, 3:-3, 3:-3, 3:-3])
