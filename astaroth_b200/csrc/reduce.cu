@@ -109,11 +109,38 @@ combine(const int op, const double a, const double b)
     return op == AC_REDUCE_OP_MAX ? fmax(a, b) : fmin(a, b);
 }
 
+constexpr int kPerLane = 4; /* cells of a row that a lane loads together */
+constexpr int kMaxBlocks = AC_SMS * 8;
+
+/* The pieces that every x row is cut into: whole rows where there is one for each warp of
+ * two blocks per SM, else pieces of a multiple of what a warp loads together, as many as
+ * those warps.  By whole rows a few long ones leave the GPU idle (20000 x 8 x 8, 64 rows:
+ * three fields 206 us, in pieces 25; 400 x 24 x 24, four fields 28 and 21); with 2400 and
+ * more rows pieces gain nothing (256 x 64 x 64 18.4 us, in two pieces 20.6). */
+struct RowPieces {
+    int length, count;
+};
+
+RowPieces
+row_pieces(const Geom& g)
+{
+    constexpr int unit      = 32 * kPerLane;
+    const long long rows    = (long long)g.ny * g.nz;
+    const long long warps   = (long long)kMaxBlocks / 4 * (kTpb / 32);
+    const long long wanted  = (warps + rows - 1) / rows;
+    const long long units   = ((long long)g.nx + unit - 1) / unit;
+    const long long count   = wanted < units ? wanted : units;
+    const long long length  = (units + count - 1) / count * unit;
+    if (count <= 1)
+        return RowPieces{g.nx, 1};
+    return RowPieces{(int)length, (int)((g.nx + length - 1) / length)};
+}
+
 /* nonfinite (optional): set to 1 when a mapped value is NaN or infinite, which a
  * maximum or minimum would otherwise hide (fmax and fmin drop NaN) */
-template <typename R>
+template <typename R, bool PIECES>
 __global__ void __launch_bounds__(kTpb)
-reduce_kernel(const Geom g, const R f, const int map, const int op,
+reduce_kernel(const Geom g, const R f, const int map, const int op, const RowPieces pc,
               double* __restrict__ partials, unsigned int* __restrict__ counter,
               double* __restrict__ result, unsigned int* __restrict__ nonfinite)
 {
@@ -123,29 +150,32 @@ reduce_kernel(const Geom g, const R f, const int map, const int op,
     const bool is_sum  = op == AC_REDUCE_OP_SUM;
     const double ident = op == AC_REDUCE_OP_MAX ? -INFINITY : INFINITY;
 
-    /* A warp takes an x row at a time, U cells per lane with their loads in flight
-     * together: a row per block with one load per thread left the kernel waiting
-     * for memory (256^3, one field: 106 -> 36 us). */
-    constexpr int U = 4;
+    /* A warp takes an x row, or a piece of one, at a time, U cells per lane with their
+     * loads in flight together: a row per block with one load per thread left the kernel
+     * waiting for memory (256^3, one field: 106 -> 36 us). */
+    constexpr int U = kPerLane;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int WARPS = kTpb / 32;
     DD acc{0.0, 0.0};
     double ext           = ident;
     bool bad             = false;
-    const long long rows = (long long)g.ny * g.nz;
-    for (long long r = (long long)blockIdx.x * WARPS + warp; r < rows;
-         r += (long long)gridDim.x * WARPS) {
+    const long long items = (long long)g.ny * g.nz * (PIECES ? pc.count : 1);
+    for (long long n = (long long)blockIdx.x * WARPS + warp; n < items;
+         n += (long long)gridDim.x * WARPS) {
+        const long long r    = PIECES ? n / pc.count : n;
+        const int first      = PIECES ? (int)(n - r * pc.count) * pc.length : 0;
+        const int end        = PIECES ? min(g.nx - first, pc.length) + first : g.nx;
         const int k          = (int)(r / g.ny);
         const int j          = (int)(r - (long long)k * g.ny);
         const long long base = geom_idx(g, NGHOST, j + NGHOST, k + NGHOST);
-        for (int i0 = lane; i0 < g.nx; i0 += 32 * U) {
+        for (int i0 = first + lane; i0 < end; i0 += 32 * U) {
             double v[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) /* past the row's end: its last cell, not used below */
-                v[u] = map_value(map, f, base + min(i0 + 32 * u, g.nx - 1));
+            for (int u = 0; u < U; ++u) /* past the end: the last cell, not used below */
+                v[u] = map_value(map, f, base + min(i0 + 32 * u, end - 1));
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                if (i0 + 32 * u >= g.nx)
+                if (i0 + 32 * u >= end)
                     continue;
                 bad |= !isfinite(v[u]);
                 if (is_sum)
@@ -235,15 +265,29 @@ reduce_kernel(const Geom g, const R f, const int map, const int op,
     }
 }
 
+template <typename R>
+void
+launch_reduce(const int blocks, cudaStream_t stream, const Geom& g, const R& f, const int map,
+              const int op, double* partials, unsigned int* counter, double* result,
+              unsigned int* nonfinite)
+{
+    const RowPieces pc = row_pieces(g);
+    if (pc.count > 1)
+        reduce_kernel<R, true>
+            <<<blocks, kTpb, 0, stream>>>(g, f, map, op, pc, partials, counter, result, nonfinite);
+    else
+        reduce_kernel<R, false>
+            <<<blocks, kTpb, 0, stream>>>(g, f, map, op, pc, partials, counter, result, nonfinite);
+}
+
 } // namespace
 
 int
 ac_reduce_blocks(const Geom& g)
 {
-    const long long rows = (long long)g.ny * g.nz;
-    const long long want = (rows + 7) / 8; /* a row per warp */
-    const long long cap  = (long long)AC_SMS * 8;
-    return (int)(want < cap ? want : cap);
+    constexpr int warps  = kTpb / 32; /* a row or a piece of one each */
+    const long long want = ((long long)g.ny * g.nz * row_pieces(g).count + warps - 1) / warps;
+    return (int)(want < kMaxBlocks ? want : kMaxBlocks);
 }
 
 cudaError_t
@@ -262,9 +306,8 @@ ac_launch_reduce(const Geom& g, const void* const* fields, const float* const* l
         Reader64 f;
         for (int q = 0; q < 4; ++q)
             f.p[q] = (const double*)fields[q < nfields ? q : 0];
-        reduce_kernel<<<blocks, kTpb, 0, stream>>>(g, f, map, op, scratch.partials,
-                                                   scratch.counter, scratch.result,
-                                                   scratch.nonfinite);
+        launch_reduce(blocks, stream, g, f, map, op, scratch.partials, scratch.counter,
+                      scratch.result, scratch.nonfinite);
     }
     else {
         ReaderComp f;
@@ -272,9 +315,8 @@ ac_launch_reduce(const Geom& g, const void* const* fields, const float* const* l
             f.hi[q] = (const float*)fields[q < nfields ? q : 0];
             f.lo[q] = lo[q < nfields ? q : 0];
         }
-        reduce_kernel<<<blocks, kTpb, 0, stream>>>(g, f, map, op, scratch.partials,
-                                                   scratch.counter, scratch.result,
-                                                   scratch.nonfinite);
+        launch_reduce(blocks, stream, g, f, map, op, scratch.partials, scratch.counter,
+                      scratch.result, scratch.nonfinite);
     }
     if (launches)
         ++*launches;
@@ -398,7 +440,7 @@ acReduceNoAlloc(const AcReal* const* fields, const int nfields, const int nx, co
     Reader64 f;
     for (int q = 0; q < 4; ++q)
         f.p[q] = fields[q < nfields ? q : 0];
-    reduce_kernel<<<nb, kTpb, 0, st>>>(g, f, map, op, partials, counter, result, nullptr);
+    launch_reduce(nb, st, g, f, map, op, partials, counter, result, nullptr);
     AC_CUDA_CHECK(cudaGetLastError());
     return AC_SUCCESS;
 }

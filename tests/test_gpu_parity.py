@@ -276,6 +276,48 @@ def test_reductions_vs_oracle(n):
             assert again == got  # deterministic
 
 
+@pytest.mark.parametrize("n", [(127, 2, 3), (128, 2, 3), (129, 2, 3), (257, 20, 10), (4099, 4, 5)])
+def test_reductions_of_long_rows(n):
+    """Rows that are cut into pieces: every cell once, the last one too, and the
+    non-finite flag wherever it is."""
+    info = ab.make_info(n, **ab.CONFIG_PARAMS)
+    f = ab.seeded_mesh(info, 9, amp_scalar=0.3, sigma_uu=0.2, sigma_aa=0.1)
+    with ab.Device(info) as dev:
+        dev.load_mesh(f)
+        for r, h in valid_reductions():
+            got = gpu_reduce(dev, r, h)
+            want = oracle.reduce(f, r, h, "port")
+            scale = magnitude_sum(f, r, h)
+            if r.endswith("RMS") or r.endswith("RMS_EXP"):
+                scale = np.sqrt(scale / np.prod(n))
+            assert abs(got - want) <= 8 * EPS * (abs(want) + scale), (r, h, got, want)
+        for x in (0, n[0] // 2, n[0] - 1):
+            g = f.copy()
+            g[1, n[2] + 2, n[1] + 2, x + 3] = 100.0 + x
+            g[2, 3, 3, x + 3] = np.nan
+            dev.load_mesh(g)
+            assert dev.reduce_scal("RTYPE_MAX", 1) == 100.0 + x and not dev.reduce_nonfinite()
+            dev.reduce_scal("RTYPE_MAX", 2)
+            assert dev.reduce_nonfinite()
+
+
+def test_reduction_time_does_not_follow_the_shape():
+    """A few long rows take about as long as a cube of as many cells."""
+    import time
+
+    times = []
+    for n in ((108, 108, 108), (19683, 8, 8)):
+        info = ab.make_info(n)
+        with ab.Device(info) as dev:
+            def once():
+                t0 = time.perf_counter()
+                dev.reduce_vec("RTYPE_RMS", 1, 2, 3)
+                return time.perf_counter() - t0
+
+            times.append(min(once() for _ in range(50)))
+    assert times[1] <= 3 * times[0], times
+
+
 @pytest.mark.parametrize("name", sorted(META["cases"]))
 def test_reductions_vs_reference_golden(name):
     info, f = case(name)
