@@ -20,9 +20,11 @@
  * gather for a vector field is - div-like first-derivative terms + lap + grad
  * div of the slot fields.  The gather runs one output field per block.
  *
- * The slot arrays hold the interior cells only, packed (x fastest, rows of nx):
- * with nx even every pair of x neighbours is then one aligned 16-byte value,
- * and adj_gather2_kernel forms two cells per thread from such loads.
+ * The slot arrays have one of two layouts (ac_adjoint_pairs).  Packed, they hold
+ * the interior cells only (x fastest, rows of nx): with nx even every pair of x
+ * neighbours is then one aligned 16-byte value, and adj_gather2_kernel forms two
+ * cells per thread from such loads.  Otherwise they are laid out as the fields,
+ * and the cells of a thread have one index in both.
  */
 #include "internal.h"
 #include "mhd_rhs_adjoint.cuh"
@@ -37,13 +39,14 @@ namespace {
  * a loop there spills its 254 registers.) */
 constexpr int KZ = 1;
 
-/* index of interior cell (i, j, k) in a slot array */
+/* index of interior cell (i, j, k) in a packed slot array */
 __device__ __forceinline__ long long
 mu_idx(const Geom& g, const int i, const int j, const int k)
 {
     return i + (long long)g.nx * (j + (long long)g.ny * k);
 }
 
+template <bool PACKED>
 __global__ void __launch_bounds__(128)
 adj_local_kernel(const Geom g, const AdjointFields a, const StencilCoef sc, const PhysConst pc,
                  const double beta, const double dt, double* __restrict__ pgrad)
@@ -56,7 +59,7 @@ adj_local_kernel(const Geom g, const AdjointFields a, const StencilCoef sc, cons
     if (i < g.nx && j < g.ny && k < g.nz) {
         const long long idx   = geom_idx(g, i + NGHOST, j + NGHOST, k + NGHOST);
         const long long st[3] = {1, (long long)g.px, g.pxy};
-        const long long midx  = mu_idx(g, i, j, k);
+        const long long midx  = PACKED ? mu_idx(g, i, j, k) : idx;
         double lam[AC_NF];
 #pragma unroll
         for (int q = 0; q < AC_NF; ++q) {
@@ -138,8 +141,8 @@ make_wrap(const Geom& g, const int i, const int j, const int k, Wrap& w)
 #pragma unroll
     for (int d = -3; d <= 3; ++d) {
         w.o[0][d + 3] = (long long)(wrap(i + d, g.nx) - i);
-        w.o[1][d + 3] = (long long)(wrap(j + d, g.ny) - j) * g.nx;
-        w.o[2][d + 3] = (long long)(wrap(k + d, g.nz) - k) * g.nx * g.ny;
+        w.o[1][d + 3] = (long long)(wrap(j + d, g.ny) - j) * g.px;
+        w.o[2][d + 3] = (long long)(wrap(k + d, g.nz) - k) * g.pxy;
     }
 }
 
@@ -220,8 +223,9 @@ gather_gd(const AdjointFields& a, const int gd0, const long long idx, const Wrap
            (sc.d2[2][0] * __ldg(g2) + wd2s<2>(g2, w, sc.d2[2]));
 }
 
-/* One output field per block (blockIdx.z = zblock * AC_NF + q), so a block
- * reads only the slot arrays of that field; KZ planes per thread. */
+/* Slot arrays laid out as the fields.  One output field per block
+ * (blockIdx.z = zblock * AC_NF + q), so a block reads only the slot arrays of
+ * that field; KZ planes per thread. */
 __global__ void __launch_bounds__(128)
 adj_gather_kernel(const Geom g, const AdjointFields a, const StencilCoef sc, const double alpha)
 {
@@ -233,28 +237,27 @@ adj_gather_kernel(const Geom g, const AdjointFields a, const StencilCoef sc, con
     const int k1 = min((int)(blockIdx.z / AC_NF + 1) * KZ, g.nz);
     for (int k = blockIdx.z / AC_NF * KZ; k < k1; ++k) {
         const long long idx = geom_idx(g, i + NGHOST, j + NGHOST, k + NGHOST);
-        const long long midx = mu_idx(g, i, j, k);
         Wrap w;
         make_wrap(g, i, j, k, w);
         double add;
         if (q == VTXBUF_LNRHO || q == VTXBUF_ENTROPY) {
             const int m = q == VTXBUF_LNRHO ? MU_L : MU_S;
-            add         = gather_gl(a, m + MU_SG, m + MU_SLAP, midx, w, sc);
+            add         = gather_gl(a, m + MU_SG, m + MU_SLAP, idx, w, sc);
         }
         else {
             const int m = q <= VTXBUF_UUZ ? MU_U : MU_A;
             const int c = q <= VTXBUF_UUZ ? q - VTXBUF_UUX : q - VTXBUF_AX;
-            add         = gather_gl(a, m + MU_VG + 3 * c, m + MU_VLAP + c, midx, w, sc);
-            add += c == 0 ? gather_gd<0>(a, m + MU_VGD, midx, w, sc)
-                          : c == 1 ? gather_gd<1>(a, m + MU_VGD, midx, w, sc)
-                                   : gather_gd<2>(a, m + MU_VGD, midx, w, sc);
+            add         = gather_gl(a, m + MU_VG + 3 * c, m + MU_VLAP + c, idx, w, sc);
+            add += c == 0 ? gather_gd<0>(a, m + MU_VGD, idx, w, sc)
+                          : c == 1 ? gather_gd<1>(a, m + MU_VGD, idx, w, sc)
+                                   : gather_gd<2>(a, m + MU_VGD, idx, w, sc);
         }
         a.lf[q][idx] += add;
         a.lw[q][idx] *= alpha;
     }
 }
 
-/* ---- two x neighbours per thread (nx even) ----
+/* ---- two x neighbours per thread (packed slot arrays, nx even) ----
  * The gather is bound by its loads through L1 (about 490 taps a cell).  As pairs a
  * row's seven x taps of both cells are 5 loads instead of 14, a y or z tap one
  * instead of two.  The sums are those of the functions above, term by term.
@@ -490,7 +493,31 @@ adj_gather2_kernel(const Geom g, const AdjointFields a, const StencilCoef sc, co
     }
 }
 
+/* the blocks of adj_gather_kernel: 32 x 4 cells of a plane and a field */
+const dim3 kTile(32, 4, 1);
+dim3
+tiles_of(const Geom& g)
+{
+    return dim3((unsigned)((g.nx + kTile.x - 1) / kTile.x), (unsigned)((g.ny + kTile.y - 1) / kTile.y),
+                (unsigned)g.nz);
+}
+
 } // namespace
+
+/* Pairs need an even nx and 32-bit offsets.  They halve the threads, which pays from about
+ * 1.75 waves of the other gather's blocks (seven per SM) on: us per adjoint substep, cells /
+ * pairs: 16^3 16.9 / 18.1, 26 x 20 x 30 (1.2 waves) 21.1 / 23.3, 28^3 (1.5) 23.0 / 24.3,
+ * 32^3 (2.0) 26.5 / 24.7, 16 x 16 x 80 (2.5) 31.6 / 27.2, 64^3 169 / 152.  With nx odd, cells of
+ * packed arrays were slower than cells of arrays like the fields' (a second set of
+ * indices, 90 registers against 72): 65 x 64 x 64 252 against 227, 95 x 79 x 80 412 / 374. */
+bool
+ac_adjoint_pairs(const Geom& g)
+{
+    const dim3 b           = tiles_of(g);
+    const long long blocks = (long long)b.x * b.y * b.z * AC_NF;
+    return g.nx % 2 == 0 && 4 * blocks >= 7 * (7LL * AC_SMS) &&
+           (long long)g.nx * g.ny * g.nz < (1LL << 31);
+}
 
 cudaError_t
 ac_launch_adjoint_substep(const Geom& g, const AdjointFields& a, const StencilCoef& sc,
@@ -498,24 +525,25 @@ ac_launch_adjoint_substep(const Geom& g, const AdjointFields& a, const StencilCo
                           const double dt, double* pgrad, cudaStream_t stream,
                           unsigned long long* launches)
 {
-    const dim3 tpb(32, 4, 1);
-    const dim3 bpg((g.nx + 31) / 32, (g.ny + 3) / 4, g.nz);
-    adj_local_kernel<<<bpg, tpb, 0, stream>>>(g, a, sc, pc, beta, dt, pgrad);
+    const dim3 bpg   = tiles_of(g);
+    const bool pairs = ac_adjoint_pairs(g);
+    if (pairs)
+        adj_local_kernel<true><<<bpg, kTile, 0, stream>>>(g, a, sc, pc, beta, dt, pgrad);
+    else
+        adj_local_kernel<false><<<bpg, kTile, 0, stream>>>(g, a, sc, pc, beta, dt, pgrad);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return e;
     const unsigned zb = (unsigned)((g.nz + KZ - 1) / KZ);
     if ((long long)zb * AC_NF > 65535)
         return cudaErrorInvalidConfiguration;
-    /* pairs where rows and arrays are 16-byte aligned (the arrays' stride is even)
-     * and 32-bit offsets reach */
-    if (g.nx % 2 == 0 && (long long)g.nx * g.ny * g.nz < (1LL << 31)) {
+    if (pairs) {
         const dim3 ppg((unsigned)((g.nx / 2 * g.ny + 127) / 128), (unsigned)g.nz * AC_NF);
         adj_gather2_kernel<<<ppg, 128, 0, stream>>>(g, a, sc, alpha);
     }
     else {
         const dim3 gpg(bpg.x, bpg.y, zb * AC_NF);
-        adj_gather_kernel<<<gpg, tpb, 0, stream>>>(g, a, sc, alpha);
+        adj_gather_kernel<<<gpg, kTile, 0, stream>>>(g, a, sc, alpha);
     }
     if (launches)
         *launches += 2;

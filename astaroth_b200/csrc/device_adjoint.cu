@@ -37,12 +37,12 @@ join_state(const Device d, cudaStream_t st, double* dst, unsigned long long* lau
     return ac_launch_fields(d->geom, field_pairs(d, p), true, st, launches);
 }
 
-/* values of one slot array: the interior cells, an even number of them */
+/* values of one slot array: the interior cells (pairs; an even number) or all cells */
 static size_t
 adj_mu_stride(const Device d)
 {
-    const size_t n = (size_t)d->geom.nx * d->geom.ny * d->geom.nz;
-    return (n + 1) / 2 * 2;
+    const Geom g = adj_geom(d);
+    return ac_adjoint_pairs(g) ? (size_t)g.nx * g.ny * g.nz : (size_t)g.cells;
 }
 
 static AcResult

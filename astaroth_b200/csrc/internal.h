@@ -391,7 +391,10 @@ cudaError_t ac_launch_cfl(const Geom& g, const FieldsT<T>& f, const StencilCoef&
                           const double cs2_sound, unsigned long long* cfl, cudaStream_t stream,
                           unsigned long long* launches);
 
-/* One adjoint substep (adjoint.cu): local reverse + halo fill of mu + gather. */
+/* Whether the adjoint's slot arrays hold the interior cells only, packed, and its gather
+ * forms two x neighbours per thread (else they are laid out as FP64 fields). */
+bool ac_adjoint_pairs(const Geom& g);
+/* One adjoint substep (adjoint.cu): local reverse, gather. */
 cudaError_t ac_launch_adjoint_substep(const Geom& g, const AdjointFields& a,
                                       const StencilCoef& sc, const PhysConst& pc,
                                       const double alpha, const double beta, const double dt,

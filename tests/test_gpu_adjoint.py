@@ -99,6 +99,44 @@ def test_adjoint_substep_matches_autograd(step):
     assert abs(eta_bar - float(geta)) <= 1e-11 * abs(float(geta))
 
 
+@pytest.mark.parametrize("n", [(4, 5, 6), (3, 4, 3), (21, 16, 12), (21, 15, 13), (33, 33, 35),
+                               (32, 32, 32), (4, 60, 120), (6, 50, 70), (96, 21, 30), (64, 16, 29)])
+@pytest.mark.parametrize("step", [1])
+def test_adjoint_substep_shapes(n, step):
+    """Both layouts of the slot arrays: small meshes and odd x sides (laid out as the
+    fields), and pairs of x neighbours, also with two or three pairs in a row, where the
+    wrapped offsets of a pair meet."""
+    torch = _torch()
+    info, f = mesh(n, 37)
+    p = ab.info_to_dict(info)
+    dt = 2e-3
+    rng = np.random.default_rng(step)
+    lam = np.zeros_like(f)
+    oracle.interior(lam)[...] = rng.standard_normal(oracle.interior(lam).shape)
+    with ab.Device(info) as dev:
+        dev.load_mesh(f)
+        dev.load_adjoint(torch.from_numpy(lam).cuda())
+        dev.integrate_substep_adjoint(step, dt)
+        # the second substep back has lw as the first one left it
+        dev.integrate_substep_adjoint(step - 1, dt)
+        out = dev.store_adjoint(torch.zeros_like(torch.from_numpy(lam)).cuda()).cpu().numpy()
+        nu_bar, eta_bar = dev.param_adjoints()
+    fi = torch.from_numpy(oracle.interior(f).copy()).requires_grad_(True)
+    nu = torch.tensor(p["nu_visc"], dtype=torch.float64, requires_grad=True)
+    eta = torch.tensor(p["eta"], dtype=torch.float64, requires_grad=True)
+    lf = torch.from_numpy(oracle.interior(lam).copy())
+    lw, want_nu, want_eta = torch.zeros_like(lf), 0.0, 0.0
+    for s in (step, step - 1):
+        lw = lw + R.BETA[s] * lf
+        g, gnu, geta = torch.autograd.grad((R.rates(fi, p, nu, eta) * (dt * lw)).sum(),
+                                           [fi, nu, eta])
+        lf, lw = lf + g, R.ALPHA[s] * lw
+        want_nu, want_eta = want_nu + float(gnu), want_eta + float(geta)
+    assert rel(oracle.interior(out), lf.numpy()) <= 1e-12
+    assert abs(nu_bar - want_nu) <= 1e-11 * abs(want_nu)
+    assert abs(eta_bar - want_eta) <= 1e-11 * abs(want_eta)
+
+
 def test_gradient_matches_cpu_reference():
     torch = _torch()
     from astaroth_b200 import autograd as AG
