@@ -12,7 +12,7 @@ whole substep of the best persistent launch with one tap-kernel launch per
 member (the same bits, the members' launches as concurrent graph branches) and,
 where some member is larger than about 96^3, with mode 1 (the launches of the
 members' own Devices), and keeps the fastest; the result can be cached in a JSON file keyed by the
-member sizes, the precision and the GPU name.
+member sizes, the precision, the GPU name and the kernels behind the modes.
 """
 from __future__ import annotations
 
@@ -55,6 +55,13 @@ def ensemble_members(n_members: int = 64, seed: int = 3, precision: int = 1,
 def _default_cache() -> Path:
     base = os.environ.get("XDG_CACHE_HOME") or os.path.join(os.path.expanduser("~"), ".cache")
     return Path(base) / "astaroth_b200" / "ensemble_tiles.json"
+
+
+# The kernels that a cached choice stands for.  It goes up when a mode takes other
+# kernels: a choice from before would give other bits than a fresh tuning (mode 1 of
+# small members was the tap kernel, with the bits of mode 0, and is the split-stage
+# kernel now).
+_FORMS = "k2"
 
 
 class Ensemble:
@@ -144,7 +151,7 @@ class Ensemble:
 
         sizes = sorted(dims(i) for i in self.infos)
         prec = self.infos[0].int_params[capi.IntParam.AC_precision]
-        return f"{torch.cuda.get_device_name()}|p{prec}|" + ",".join(
+        return f"{torch.cuda.get_device_name()}|p{prec}|{_FORMS}|" + ",".join(
             f"{a}x{b}x{c}" for a, b, c in sizes)
 
     def autotune(self, cache: str | os.PathLike | None = None, use_cache: bool = True):

@@ -112,6 +112,30 @@ def test_autotune_keeps_state_and_results(tmp_path):
         assert np.array_equal(got[m], ref(infos[m], seeds[m], 1))
 
 
+def test_autotune_passes_over_choices_for_other_kernels(tmp_path):
+    """A cache written when mode 1 was the tap kernel (its key had no mark of the kernels)
+    is not replayed: the step keeps the bits of the sequential launches."""
+    import json
+
+    import torch
+
+    infos, seeds = _members(1, [32, 48, 64])
+    cache = tmp_path / "tiles.json"
+    old = torch.cuda.get_device_name() + "|p1|32x32x32,48x48x48,64x64x64"
+    cache.write_text(json.dumps({old: [32, 4, 8, 0, 1]}))
+    with Ensemble(infos) as e:
+        e.load_seeded(seeds)
+        e.set_timesteps(DT)
+        tiles, ms = e.autotune(cache=cache)
+        assert ms is not None and tiles[4] == 0
+        e.integrate_step()
+        e.synchronize()
+        got = [e.store_member(m) for m in range(e.n)]
+    assert set(json.loads(cache.read_text())) > {old}  # other entries stay
+    for m in range(len(infos)):
+        assert np.array_equal(got[m], _device_run(infos[m], seeds[m], 1))
+
+
 def _device_tiled(info, seed, steps):
     with Device(info) as d:
         d.load_mesh(seeded_mesh(info, seed))
