@@ -3,7 +3,9 @@
  * (FP64 meshes), or two floats of two cells with the same x (FP32 compensated
  * meshes) that move through packed FP32x2 instructions, so that both
  * precisions have 64-bit values and one instruction stream.  Multiply-adds are
- * written out (vfma): packed operations are never contracted by the compiler.
+ * written out (vfma).  A packed product may all the same be fused with a packed sum
+ * that follows it; where the rounded product itself is needed (the increment of the
+ * RK update), it is formed by scalar products.
  */
 #pragma once
 

@@ -202,8 +202,11 @@ def cpu_reference_sample(n: int, steps: int = 1):
     dt = time.perf_counter() - t0
     cores = int(os.environ.get("OMP_NUM_THREADS", os.cpu_count() or 1))
     return {"value": n ** 3 * steps / dt, "unit": UNIT, "cores": cores, "kind": kind,
-            "sample": f"{steps} RK3 step(s) of the reference host model "
-                      f"(src/utils/modelsolver.cc acHostIntegrateStep, long double, OpenMP) "
+            "sample": f"{steps} RK3 step(s) of "
+                      + ("the reference host model (src/utils/modelsolver.cc "
+                         "acHostIntegrateStep, " if kind == "reference" else
+                         "this project's C restatement of the reference host model (")
+                      + f"long double, OpenMP) "
                       f"on a {n}^3 periodic box, same physics and seeded distributions; "
                       f"rate per cell",
             "seconds": dt}

@@ -99,8 +99,8 @@ typedef enum {
     /* Selects the solve kernel (for tests and timing): 0 = the default (the
      * split-stage kernel where it takes the mesh, but for small FP64 meshes with
      * an odd x side, else the per-plane tap kernel, else the plain one), 1 = the plain (untiled) kernel, 2 = the tiled kernel
-     * that reads every stencil tap of plane z from shared memory, 3 and 4 = the
-     * split-stage kernel for every mesh that it takes. */
+     * that reads every stencil tap of plane z from shared memory, 3 (and 4) =
+     * the split-stage kernel for every mesh that it takes. */
     AC_debug_plain_kernel,
     /* Upwinding terms of the continuity and momentum equations when nonzero:
      * the reference's LUPWD build option (mhdsolver.ac:101,336-338,357-359;

@@ -33,12 +33,12 @@ def clean_step(info, f, kernel):
         return dev.store_mesh()
 
 
-@pytest.mark.parametrize("precision", [0, 1])
-# the leading-plane kernel with the group exchange through tensor memory or
-# shared memory, the per-plane tap kernel
-@pytest.mark.parametrize("kernel", [3, 4, 2])
-def test_bounded_wait_gives_up_and_device_recovers(precision, kernel):
-    info = ab.make_info((64, 16, 40), precision=precision, **ab.CONFIG_PARAMS)
+# the split-stage kernel with planes by TMA and (FP64, nx odd) by its threads, the
+# per-plane tap kernel
+@pytest.mark.parametrize("kernel,nx,precision", [(3, 64, 0), (3, 64, 1), (3, 65, 0), (2, 64, 0),
+                                                 (2, 64, 1)])
+def test_bounded_wait_gives_up_and_device_recovers(kernel, nx, precision):
+    info = ab.make_info((nx, 16, 40), precision=precision, **ab.CONFIG_PARAMS)
     f = ab.seeded_mesh(info, 3)
     lib = capi.load()
     with ab.Device(info) as dev:

@@ -34,13 +34,11 @@ def _interior(a):
 
 # overlap: the interior planes solved while the planes travel, then the ends
 @pytest.mark.parametrize("overlap", [False, True])
-@pytest.mark.parametrize("kernel", [0, 3])  # the default choice; the leading-plane kernel
+@pytest.mark.parametrize("kernel", [0, 3])  # the default choice; the split-stage kernel
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("shape,slabs", [((40, 36, 48), 2), ((32, 32, 20), 3), ((40, 36, 48), 4),
                                          ((33, 24, 16), 1)])
 def test_slabs_equal_one_device(shape, slabs, precision, kernel, overlap):
-    if kernel == 3 and (precision == 0 and shape[0] % 2):
-        pytest.skip("odd nx in FP64 takes the plain kernel")
     info = make_info(shape, precision=precision)
     info.int_params[IntParam.AC_debug_plain_kernel] = kernel
     f = seeded_mesh(info, 81)
