@@ -60,6 +60,7 @@
  */
 #include <cuda.h>
 #include <atomic>
+#include <initializer_list>
 #include <type_traits>
 #include <vector>
 
@@ -123,11 +124,12 @@ struct SplitMaps {
 template <typename V>
 struct SplitCoef {
     V d1[3][3];  /* first derivative, [axis][k-1] */
-    /* Laplacians of lnrho and s, and of A, each in a unit of its own (lap_unit; FP64: 1)
-     * that the factors gicp_l, gm1_l and eta, nim take back: sides, [axis][k-1]; centres of
-     * all axes; A: centres of two axes, and what av_c[a] adds to that of the other two */
-    V sd2[3][3], s_all;
-    V ad2[3][3], a_xy, a_yz, a_xz, av_c[3];
+    /* Laplacians of lnrho, s and A in a unit (lap_unit; FP64: 1) that the factors gicp_l,
+     * gm1_l, eta and nim take back: sides, [axis][k-1]; what d2c[a] adds to the centre of
+     * the other two axes; centres of all axes and of two */
+    V d2[3][3];
+    V d2c[3];
+    V c_all, c_xy, c_yz, c_xz;
     /* hydro: nu lap u_c + vg d/dx_c div u, vg = nu/3 + zeta */
     V vd[3][3]; /* (nu + vg) d2 sides: axis c of component c */
     V vn[3][3]; /* nu d2 sides: the other axes */
@@ -140,7 +142,7 @@ struct SplitCoef {
     /* magnetic: j = (grad div A - lap A) / mu0 */
     V mm[3][3]; /* mix / mu0 */
     V mmn[2][3];
-    V nim;      /* -1/mu0, in the unit of lap A */
+    V nim;      /* -1/mu0 (times lap_unit) */
     V up[3][4]; /* upwinding, [axis][k]: centre and sides */
     /* equations */
     V m23, two, one_half, nu, inv_cp, ncs2, gicp, gm1, gicp_l, gm1_l, gm1_lnrho0, inv_exp_lnT0, eta,
@@ -155,21 +157,24 @@ made_up(const double v)
     return r > 0.5 && r < 2 ? r : 1; /* (1 for zero and for what FP32 does not hold) */
 }
 
-/* FP32: a unit for Laplacians that are only used times fa and fb.  The sides of an
- * isotropic mesh are 270, -27 and 2 in units of 1/(180 dx^2) and the centre is -1470, so
- * that in 1/m of it, m a whole number, all of them are FP32 numbers and a constant has no
- * Laplacian: only fa and fb times the unit are rounded, and m is the one of 32 for which
- * these are rounded least (to about 5e-9 of themselves).  Rounded at 1/ds^2 every
- * coefficient was off by up to 6e-8, by chance of the spacing, and a constant had a
- * Laplacian of 5e-7 / ds^2 of its value at 512^3 (entropy 3.0e-7 off FP64 after 100 steps). */
+/* FP32: a unit for Laplacians that are only used times the factors f.  The sides of an
+ * isotropic mesh are 270, -27 and 2 in units of 1/(180 ds^2) and the centre is -1470, so
+ * that in 1/m of it (ds: the smallest spacing), m a whole number, all of them are FP32
+ * numbers and a constant has no Laplacian: only the factors times the unit are rounded, and
+ * m is the one of 64 for which these are rounded least (to about 1.5e-8 of themselves).
+ * Rounded at 1/ds^2 every coefficient was off by up to 6e-8, by chance of the spacing, and a
+ * constant had a Laplacian of 5e-7 / ds^2 of its value at 512^3 (entropy 3.0e-7 off FP64
+ * after 100 steps). */
 inline long double
-lap_unit(const StencilCoef& s, const double fa, const double fb)
+lap_unit(const StencilCoef& s, const std::initializer_list<double> f)
 {
-    const double base = s.d2[0][1] / 270;
+    const double base = fmax(s.d2[0][1], fmax(s.d2[1][1], s.d2[2][1])) / 270;
     double least      = 1;
     int best          = 1;
-    for (int m = 1; m <= 32; ++m) {
-        const double off = fmax(fabs(made_up(fa * base / m) - 1), fabs(made_up(fb * base / m) - 1));
+    for (int m = 1; m <= 64; ++m) {
+        double off = 0;
+        for (const double v : f)
+            off = fmax(off, fabs(made_up(v * base / m) - 1));
         if (off < least) {
             least = off;
             best  = m;
@@ -189,18 +194,17 @@ make_coef(const StencilCoef& s, const PhysConst& p, const RkCoef& rk)
      * the rates that are rounded anyhow make up for that, and ab for beta's part (lnrho,
      * whose rate has no factors, keeps the rounding of dt).  With it u, A and s end a run half
      * as far off FP64, over the sizes and options of 44 runs (100 steps at 512^3: u 1.0e-7,
-     * A 5.9e-8, s 7.9e-8; each factor rounded by itself 1.4e-7, 3.5e-7, 3.0e-7) */
+     * A 5.9e-8, s 7.1e-8; each factor rounded by itself 1.4e-7, 3.5e-7, 3.0e-7) */
     const double t = FP32 ? made_up(rk.beta) * made_up(rk.dt) : 1;
     const long double nu = p.nu * t, vg = ((long double)p.nu / 3 + p.zeta) * t, im = p.inv_mu0;
     /* K multiplies the Laplacians of lnrho and s too: their factors make up for its rounding */
     const double kr      = FP32 ? made_up(p.K * t) : 1;
-    const long double us = FP32 ? lap_unit(s, p.gamma_inv_cp * kr, p.gamma_m1 * kr) : 1;
-    const long double ua = FP32 ? lap_unit(s, p.eta * t, p.inv_mu0) : 1;
+    const long double unit =
+        FP32 ? lap_unit(s, {p.gamma_inv_cp * kr, p.gamma_m1 * kr, p.eta * t, p.inv_mu0}) : 1;
     for (int a = 0; a < 3; ++a) {
         for (int k = 0; k < 3; ++k) {
             c.d1[a][k] = D(s.d1[a][k]);
-            c.sd2[a][k] = D(s.d2[a][k + 1] / us);
-            c.ad2[a][k] = D(s.d2[a][k + 1] / ua);
+            c.d2[a][k] = D(s.d2[a][k + 1] / unit);
             c.vd[a][k] = D((nu + vg) * s.d2[a][k + 1]);
             c.vn[a][k] = D(nu * s.d2[a][k + 1]);
             c.vm[a][k] = D(vg * s.mix[a][k]);
@@ -228,24 +232,24 @@ make_coef(const StencilCoef& s, const PhysConst& p, const RkCoef& rk)
     /* centres: FP64 the sums of the three axes'; FP32 minus the sums of the rounded sides,
      * rounded once (they differ where the spacings do) */
     auto in_T    = [](const long double v) { return (long double)(typename Pack<V>::T)(double)v; };
-    auto centre  = [&](const int a, const long double u) {
-        long double v = s.d2[a][0];
+    long double ctr[3];
+    for (int a = 0; a < 3; ++a) {
+        ctr[a] = s.d2[a][0];
         if (FP32) {
-            v = 0;
+            ctr[a] = 0;
             for (int k = 1; k <= 3; ++k)
-                v -= 2 * in_T(s.d2[a][k] / u);
+                ctr[a] -= 2 * in_T(s.d2[a][k] / unit);
         }
-        return v;
-    };
-    const long double ax = centre(0, ua), ay = centre(1, ua), az = centre(2, ua);
-    c.s_all = D(centre(0, us) + centre(1, us) + centre(2, us));
-    c.a_xy  = D(ax + ay);
-    c.a_yz  = D(ay + az);
-    c.a_xz  = D(ax + az);
-    c.av_c[0] = D(FP32 ? ax + ay + az - in_T(ay + az) : ax);
-    c.av_c[1] = D(FP32 ? ax + ay + az - in_T(ax + az) : ay);
-    c.av_c[2] = D(FP32 ? ax + ay + az - in_T(ax + ay) : az);
-    c.nim          = D(-im * ua);
+    }
+    const long double all = ctr[0] + ctr[1] + ctr[2];
+    c.c_all = D(all);
+    c.c_xy  = D(ctr[0] + ctr[1]);
+    c.c_yz  = D(ctr[1] + ctr[2]);
+    c.c_xz  = D(ctr[0] + ctr[2]);
+    c.d2c[0] = D(FP32 ? all - in_T(ctr[1] + ctr[2]) : ctr[0]);
+    c.d2c[1] = D(FP32 ? all - in_T(ctr[0] + ctr[2]) : ctr[1]);
+    c.d2c[2] = D(FP32 ? all - in_T(ctr[0] + ctr[1]) : ctr[2]);
+    c.nim          = D(-im * unit);
     c.m23          = D(-2.0L / 3);
     c.two          = D(2);
     c.one_half     = D(0.5);
@@ -254,11 +258,11 @@ make_coef(const StencilCoef& s, const PhysConst& p, const RkCoef& rk)
     c.ncs2         = D(-p.cs2_sound * t);
     c.gicp         = D(p.gamma_inv_cp);
     c.gm1          = D(p.gamma_m1);
-    c.gicp_l       = D(p.gamma_inv_cp * kr * us);
-    c.gm1_l        = D(p.gamma_m1 * kr * us);
+    c.gicp_l       = D(p.gamma_inv_cp * kr * unit);
+    c.gm1_l        = D(p.gamma_m1 * kr * unit);
     c.gm1_lnrho0   = D(-(long double)p.gamma_m1 * p.lnrho0);
     c.inv_exp_lnT0 = D(p.inv_exp_lnT0);
-    c.eta          = D(p.eta * t * ua);
+    c.eta          = D(p.eta * t * unit);
     c.eta_mu0      = D(p.eta_mu0 * t);
     c.zeta         = D(p.zeta * t);
     c.K            = D(p.K * t);
@@ -551,7 +555,7 @@ inplane_role(const SplitMaps* maps, const SplitCoef<V>& c, const Chunk& ch,
                 upwind(0, vs);
                 r.set(H_SX, dot3(dx, c.d1[0]));
                 r.set(H_SY, dot3(dy, c.d1[1]));
-                r.set(H_SL, dot3p(sy, c.sd2[1], dot3p(sx, c.sd2[0], c.s_all * vs)));
+                r.set(H_SL, dot3p(sy, c.d2[1], dot3p(sx, c.d2[0], c.c_all * vs)));
                 taps_xy(t0, dx, sx, dy, sy);
                 upwind(1, v0);
                 const V done = mixed_first(acc[2], dx, e1, n1);
@@ -580,27 +584,27 @@ inplane_role(const SplitMaps* maps, const SplitCoef<V>& c, const Chunk& ch,
                 taps_xy(ts, dx, sx, dy, sy);
                 set(M_SX, dot3(dx, c.d1[0]));
                 set(M_SY, dot3(dy, c.d1[1]));
-                set(M_SL, dot3p(sy, c.sd2[1], dot3p(sx, c.sd2[0], c.s_all * vs)));
+                set(M_SL, dot3p(sy, c.d2[1], dot3p(sx, c.d2[0], c.c_all * vs)));
                 taps_xy(t0, dx, sx, dy, sy);
                 const V done = mixed_first(acc[2], dx, e1, n1);
                 const V dyAx = dot3(dy, c.d1[1]);
                 {
-                    const V Y = dot3p(sy, c.ad2[1], c.a_yz * v0);
-                    set(M_L0, dot3p(sx, c.ad2[0], vfma(c.av_c[0], v0, Y)));
+                    const V Y = dot3p(sy, c.d2[1], c.c_yz * v0);
+                    set(M_L0, dot3p(sx, c.d2[0], vfma(c.d2c[0], v0, Y)));
                     set(M_Q0, dxy(t1, c.mm[0], c.nim * Y));
                 }
                 taps_xy(t1, dx, sx, dy, sy);
                 fin.set(2, mixed_second(acc[2], done, dy, e2, n2));
                 {
-                    const V X = dot3p(sx, c.ad2[0], c.a_xz * v1);
-                    set(M_L1, dot3p(sy, c.ad2[1], vfma(c.av_c[1], v1, X)));
+                    const V X = dot3p(sx, c.d2[0], c.c_xz * v1);
+                    set(M_L1, dot3p(sy, c.d2[1], vfma(c.d2c[1], v1, X)));
                     set(M_Q1, dxy(t0, c.mm[0], c.nim * X));
                 }
                 set(M_BZ, dot3(dx, c.d1[0]) - dyAx);
                 taps_xy(t2, dx, sx, dy, sy);
                 fin.set(0, mixed_first(acc[0], dx, e1, n1));
                 fin.set(1, mixed_first(acc[1], dy, e2, n2));
-                set(M_L2, dot3p(sy, c.ad2[1], dot3p(sx, c.ad2[0], c.a_xy * v2)));
+                set(M_L2, dot3p(sy, c.d2[1], dot3p(sx, c.d2[0], c.c_xy * v2)));
                 set(M_DXAZ, dot3(dx, c.d1[0]));
                 set(M_DYAZ, dot3(dy, c.d1[1]));
                 __syncwarp();
@@ -880,7 +884,7 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
             const V lnrho = w[3].template get<V>(0), ux = w[3].template get<V>(1), uy = w[3].template get<V>(2),
                     uz = w[3].template get<V>(3);
             V gl[3], gz[3], s2[4];
-            z_derivs(w, 0, c.d1[2], c.sd2[2], gl[2], s2[0]);
+            z_derivs(w, 0, c.d1[2], c.d2[2], gl[2], s2[0]);
             z_derivs(w, 1, c.d1[2], c.vn[2], gz[0], s2[1]);
             z_derivs(w, 2, c.d1[2], c.vn[2], gz[1], s2[2]);
             z_derivs(w, 3, c.d1[2], c.vd[2], gz[2], s2[3]);
@@ -985,10 +989,10 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
             uw.load(ch.tl + TM::ZQ0 + (uint32_t)(p & 7) * ZQ_W);
             const V ent = w[3].template get<V>(0);
             V gs[3], s2[4], dzAx, dzAy, unused;
-            z_derivs(w, 0, c.d1[2], c.sd2[2], gs[2], s2[0]);
-            z_derivs(w, 1, c.d1[2], c.ad2[2], dzAx, s2[1]);
-            z_derivs(w, 2, c.d1[2], c.ad2[2], dzAy, s2[2]);
-            z_derivs(w, 3, c.d1[2], c.ad2[2], unused, s2[3]);
+            z_derivs(w, 0, c.d1[2], c.d2[2], gs[2], s2[0]);
+            z_derivs(w, 1, c.d1[2], c.d2[2], dzAx, s2[1]);
+            z_derivs(w, 2, c.d1[2], c.d2[2], dzAy, s2[2]);
+            z_derivs(w, 3, c.d1[2], c.d2[2], unused, s2[3]);
             val[0] = w[3].template get<V>(1);
             val[1] = w[3].template get<V>(2);
             val[2] = w[3].template get<V>(3);
@@ -1008,7 +1012,7 @@ solve_role(const Geom& g, const RoleFields<typename Pack<V>::T>& f, const SplitC
             const V j1 = vfma(c.nim, s2[2], R(M_Q1) + a.template get<V>(1));
             const V j2 = vfma(c.nim, l2, a.template get<V>(2));
             const V lap0 = R(M_L0) + s2[1], lap1 = R(M_L1) + s2[2];
-            const V lap2 = l2 + vfma(c.av_c[2], val[2], s2[3]);
+            const V lap2 = l2 + vfma(c.d2c[2], val[2], s2[3]);
             {
                 TWords<MX_N> xw;
                 xw.set(0, gs[0]);
