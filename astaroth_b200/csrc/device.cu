@@ -715,8 +715,27 @@ acDeviceResetMesh(const Device d, const Stream stream)
 /* ---- integration ---- */
 
 
+/* FP32: the update adds beta (dt rate + ab (f - f_prev)), each factor rounded.  Its bracket
+ * may have any unit, and has the one in which the roundings of beta and ab, the same in
+ * every step, are least (about 1e-9; as they are, up to 5e-8, which with dt's made 7.5e-8
+ * of all that changes in a run at dt = 1e-3).  The unit is the substep's, whatever dt is. */
+static double
+rk_unit(const double beta, const double ab)
+{
+    auto off = [](const double v) { return v != 0 ? fabs((double)(float)v / v - 1) : 0.0; };
+    double best = 1, least = 1;
+    for (int m = 0; m < 1024; ++m) {
+        const double u = 1 + m / 1024.0, o = fmax(off(beta / u), off(ab * u));
+        if (o < least) {
+            least = o;
+            best  = u;
+        }
+    }
+    return best;
+}
+
 RkCoef
-ac_rk_coef(const int step, const double dt)
+ac_rk_coef(const int step, const double dt, const int precision)
 {
     /* Williamson 2N RK3, acc-runtime/stdlib/integrators.h:11-13 */
     const double alpha[3] = {0.0, -5.0 / 9.0, -153.0 / 128.0};
@@ -726,6 +745,13 @@ ac_rk_coef(const int step, const double dt)
     rk.dt   = dt;
     rk.beta = beta[step];
     rk.ab   = step == 0 ? 0.0 : alpha[step] / beta[step - 1];
+    if (precision != 0) {
+        static const double unit[3] = {rk_unit(beta[0], 0), rk_unit(beta[1], alpha[1] / beta[0]),
+                                       rk_unit(beta[2], alpha[2] / beta[1])};
+        rk.dt *= unit[step];
+        rk.beta /= unit[step];
+        rk.ab *= unit[step];
+    }
     return rk;
 }
 
@@ -754,7 +780,7 @@ launch_substep(Device d, cudaStream_t st, const int step, const double dt,
     }
     if (step == 2)
         forcing_for_launch(d->config, dt, &pc);
-    const RkCoef rk = ac_rk_coef(step, dt);
+    const RkCoef rk = ac_rk_coef(step, dt, d->precision);
     if (step == 2 && first_box && d->config.int_params[AC_lbfield] && d->bfield) {
         /* B = curl A of this substep's input (the in-buffer is not written) */
         const void* a[3];

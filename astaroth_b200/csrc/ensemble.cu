@@ -87,7 +87,7 @@ ens_solve_kernel(const EnsMember<T>* __restrict__ mem, const int4* __restrict__ 
             cur = it.x;
         }
         RkCoef r = rk;
-        r.dt     = dt;
+        r.dt     = dt * rk.dt; /* (rk.dt: the substep's unit) */
         const BlockFieldsT<T> bf = f;
         const int i = it.y + lx, j = it.z + ly;
         if (i < g.nx && j < g.ny) {
@@ -348,7 +348,7 @@ tiles_ok(const AcEnsembleTiles t)
 cudaError_t
 launch_solve(Ensemble e, const int step, unsigned long long* launches)
 {
-    const RkCoef rk = ac_rk_coef(step, 0.0); /* dt comes from the device array */
+    const RkCoef rk = ac_rk_coef(step, 1.0, e->precision); /* dt comes from the device array */
     const int threads = e->tiles.tx * e->tiles.ty;
     if (e->precision == 0)
         ens_solve_kernel<double, false><<<e->grid, threads, 0, e->stream>>>(
@@ -418,7 +418,7 @@ record_members(Ensemble e, const int s0, const int s1, unsigned long long* launc
                 if (err != cudaSuccess)
                     return err;
             }
-            const RkCoef rk     = ac_rk_coef(s, e->dts[m]);
+            const RkCoef rk     = ac_rk_coef(s, e->dts[m], e->precision);
             const void* tmap    = &e->tmaps[2 * m + p];
             /* the kernel a Device of this member would use, or (exact) one with the
              * plain kernel's bits.  The members of the
@@ -504,7 +504,7 @@ sequential_step(Ensemble e)
                                                     e->stream, &e->launches);
             if (err != cudaSuccess)
                 return err;
-            const RkCoef rk = ac_rk_coef(s, e->dts[m]);
+            const RkCoef rk = ac_rk_coef(s, e->dts[m], e->precision);
             if constexpr (COMP)
                 err = ac_launch_solve_plain32(r.g, f, e->sc[m], e->pc[m], rk, nullptr, e->stream,
                                               &e->launches);

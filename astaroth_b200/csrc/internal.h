@@ -101,7 +101,8 @@ stencil_cast(const StencilCoef& s)
 /* Coefficients of one substep of the 2N RK3 scheme in single-pass form
  * (acc-runtime/stdlib/integrators.h:11-29):
  *   f_new = f + beta_s * (ab * (f - f_prev) + dt * rate),  ab = alpha_s / beta_{s-1}
- * with ab = 0 at s = 0 (f_prev is then not read). */
+ * with ab = 0 at s = 0 (f_prev is then not read).  For FP32 meshes dt and ab are
+ * multiplied and beta is divided by the substep's unit (ac_rk_coef). */
 struct RkCoef {
     double beta;
     double ab;
@@ -406,4 +407,4 @@ void ac_make_stencil(const AcMeshInfo& info, StencilCoef* sc);
 void ac_make_phys(const AcMeshInfo& info, PhysConst* pc);
 Geom ac_make_geom(const AcMeshInfo& info, const int precision);
 /* Coefficients of RK3 substep `step` (0, 1, 2) with timestep dt. */
-RkCoef ac_rk_coef(const int step, const double dt);
+RkCoef ac_rk_coef(const int step, const double dt, const int precision);

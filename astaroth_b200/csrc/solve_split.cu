@@ -136,7 +136,7 @@ struct SplitCoef {
     V vc[3];    /* the centre of component c, all axes */
     V vcl[3];   /* FP32: what vc lacks to cancel the sides exactly.  Rounded to FP32 alone it
                  * changes a constant u by up to 6e-8 of itself per nu/ds^2 of time, in one
-                 * direction (512^3, 100 steps: 1.6e-6 of max|u|; with this 1.3e-7) */
+                 * direction (512^3, 100 steps: 1.6e-6 of max|u|; with this 1.1e-7) */
     V vm[3][3]; /* vg mix, [xy, xz, yz][k-1] */
     V vmn[2][3]; /* -vg mix, [xz, yz] */
     /* magnetic: j = (grad div A - lap A) / mu0 */
@@ -185,22 +185,20 @@ lap_unit(const StencilCoef& s, const std::initializer_list<double> f)
 
 template <typename V>
 SplitCoef<V>
-make_coef(const StencilCoef& s, const PhysConst& p, const RkCoef& rk)
+make_coef(const StencilCoef& s, const PhysConst& p)
 {
     SplitCoef<V> c;
     auto D          = [](const long double v) { return Pack<V>::dup((double)v); };
     constexpr bool FP32 = Pack<V>::N == 2;
-    /* FP32: an increment is beta dt times a rate, beta and dt each rounded.  The factors of
-     * the rates that are rounded anyhow make up for that, and ab for beta's part (lnrho,
-     * whose rate has no factors, keeps the rounding of dt).  With it u, A and s end a run half
-     * as far off FP64, over the sizes and options of 44 runs (100 steps at 512^3: u 1.0e-7,
-     * A 5.9e-8, s 7.1e-8; each factor rounded by itself 1.4e-7, 3.5e-7, 3.0e-7) */
-    const double t = FP32 ? made_up(rk.beta) * made_up(rk.dt) : 1;
-    const long double nu = p.nu * t, vg = ((long double)p.nu / 3 + p.zeta) * t, im = p.inv_mu0;
+    const long double nu = p.nu, vg = (long double)p.nu / 3 + p.zeta, im = p.inv_mu0;
     /* K multiplies the Laplacians of lnrho and s too: their factors make up for its rounding */
-    const double kr      = FP32 ? made_up(p.K * t) : 1;
+    const double kr      = FP32 ? made_up(p.K) : 1;
     const long double unit =
-        FP32 ? lap_unit(s, {p.gamma_inv_cp * kr, p.gamma_m1 * kr, p.eta * t, p.inv_mu0}) : 1;
+        FP32 ? lap_unit(s, {p.gamma_inv_cp * kr, p.gamma_m1 * kr, p.eta, p.inv_mu0}) : 1;
+    /* The heating eta mu0 j^2 / rho + 2 nu S:S + zeta (div u)^2 is used times exp(-lnT0) only:
+     * that factor makes up for the rounding of nu, the others for what it then is off */
+    const double by_T = FP32 ? p.inv_exp_lnT0 * made_up(p.nu) : p.inv_exp_lnT0;
+    const double rest = FP32 ? made_up(by_T) / made_up(p.nu) : 1;
     for (int a = 0; a < 3; ++a) {
         for (int k = 0; k < 3; ++k) {
             c.d1[a][k] = D(s.d1[a][k]);
@@ -255,17 +253,17 @@ make_coef(const StencilCoef& s, const PhysConst& p, const RkCoef& rk)
     c.one_half     = D(0.5);
     c.nu           = D(nu);
     c.inv_cp       = D(p.inv_cp);
-    c.ncs2         = D(-p.cs2_sound * t);
+    c.ncs2         = D(-p.cs2_sound);
     c.gicp         = D(p.gamma_inv_cp);
     c.gm1          = D(p.gamma_m1);
     c.gicp_l       = D(p.gamma_inv_cp * kr * unit);
     c.gm1_l        = D(p.gamma_m1 * kr * unit);
     c.gm1_lnrho0   = D(-(long double)p.gamma_m1 * p.lnrho0);
-    c.inv_exp_lnT0 = D(p.inv_exp_lnT0);
-    c.eta          = D(p.eta * t * unit);
-    c.eta_mu0      = D(p.eta_mu0 * t);
-    c.zeta         = D(p.zeta * t);
-    c.K            = D(p.K * t);
+    c.inv_exp_lnT0 = D(by_T);
+    c.eta          = D(p.eta * unit);
+    c.eta_mu0      = D(p.eta_mu0 * rest);
+    c.zeta         = D(p.zeta * rest);
+    c.K            = D(p.K);
     return c;
 }
 
@@ -1275,11 +1273,11 @@ launch_split(const Geom& g, const SplitMaps& tm, const FieldsT<T>& f, const Sten
     const int zc = split_zchunk(bx * by, nzr, sms);
     const dim3 bpg(bx, by, (nzr + zc - 1) / zc);
     const dim3 tpb(TX, ROLES * WARPS_Y, 1);
-    const SplitCoef<V> c = make_coef<V>(sc, pc, rk);
+    const SplitCoef<V> c = make_coef<V>(sc, pc);
     RkV<V> r;
     r.dt   = Pack<V>::dup(rk.dt);
     r.beta = Pack<V>::dup(rk.beta);
-    r.ab   = Pack<V>::dup(Pack<V>::N == 2 ? rk.ab * made_up(rk.beta) : rk.ab);
+    r.ab   = Pack<V>::dup(rk.ab);
     const bool sum = pc.cfl_sum != 0, skip = pc.debug_skip_load != 0;
     cudaError_t e = cudaSuccess;
     auto launch = [&](auto kernel) {
