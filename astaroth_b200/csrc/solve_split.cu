@@ -34,10 +34,10 @@
  * no slot is written while it is read.
  *
  * What bounds it (B200, 256^3): FP64 issues on 68% of cycles with the FP64 pipe
- * 52% busy and shared memory 62%; FP32 issues on 67%.  One warp of every role
+ * 55% busy and shared memory 65%; FP32 issues on 63-66%.  One warp of every role
  * per scheduler keeps all of these in use at once; two groups of one kind
  * (one barrier per plane, 8 warps) issued on 59%.  Measured against that kernel,
- * per RK3 step: 256^3 FP64 3.60 -> 3.01 ms, FP32 3.09 -> 2.44 ms; 128^3 0.60 ->
+ * per RK3 step: 256^3 FP64 3.60 -> 3.01 ms, FP32 3.09 -> 2.5 ms; 128^3 0.60 ->
  * 0.46 and 0.50 -> 0.36 ms.  A barrier per quarter instead of the block's lets
  * the roles drift apart, and the instruction cache then misses (FP32 0.98 -> 1.18
  * ms a substep); a fifth role for uz, Az and the scalars takes the registers
